@@ -204,7 +204,7 @@ struct SortPlan {
     bool msd;
     int msd_passes;
     int msd_lo_bits;           // key 0 bits ranked directly in runs (below the shared-memory passes)
-    uint32_t msd_cap;          // rows a chunk may hold (kMsdCap, or kMsdWideCap)
+    uint32_t msd_cap;          // rows a chunk may hold (kMsdCap or kMsdWideCap)
     uint32_t msd_chunk_rows;   // nominal rows per chunk
     uint32_t msd_chunks;       // ceil(n / msd_chunk_rows)
     size_t off_msd_hist, off_msd_offs, off_msd_flag, off_chunks;
@@ -258,6 +258,7 @@ struct MsdLocalArgs {
     const void* sec;         // raw key 1 column (null for one key)
     int sec_dtype, dtype, invert, reverse;
     uint32_t lo_bits;        // key 0 bits below the shared-memory passes
+    uint32_t pshift;         // key >> pshift: the bits the rows are sorted by (segmented: per chunk)
     uint32_t* flag;
     uint32_t* err;
     void* keys_out;          // raw sorted key 0 (may be null)

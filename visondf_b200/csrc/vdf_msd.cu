@@ -23,18 +23,18 @@
 //                    [c*T, (c+1)*T); found by a two-level warp search for
 //                    the first bucket boundary at or after c*T
 //   5. k_msd_local   one CTA per chunk (<= kMsdCap rows): one counting pass
-//                    over 8192 bins of (key - chunk minimum) >> S puts the
-//                    rows of spread keys about one per bin; the rows sharing
-//                    a bin are ranked by (key 0, key 1's order image,
-//                    position in the chunk) -- key 1 is read through the row
-//                    id only where key 0 ties -- and the raw sorted key 0 and
-//                    the permutation are written.  A chunk where a bin holds
-//                    a run longer than kMsdRunMax (many equal or clustered
-//                    keys) is sorted instead by stable 8-bit LSD passes in
-//                    shared memory over the digits of key 0 above its low F
-//                    bits that vary inside it, with runs of equal high bits
-//                    ranked the same way (F = 32 for 8-byte keys, 0 for
-//                    4-byte keys).
+//                    over kMsdCap bins of the chunk's key range puts the rows
+//                    of spread keys about two bins apart; the rows sharing a
+//                    bin are ranked by (key 0, key 1's order image, position
+//                    in the chunk) -- key 1 is read through the row id only
+//                    where key 0 ties -- and the raw sorted key 0 and the
+//                    permutation are written.  A chunk where a bin holds a
+//                    run longer than kMsdRunMax (many equal or clustered
+//                    keys) is sorted instead by stable passes over the dense
+//                    bin index, or by stable 8-bit LSD passes in shared
+//                    memory over the digits of key 0 above its low F bits
+//                    that vary inside it, with runs of equal high bits ranked
+//                    the same way (F = 32 for 8-byte keys, 0 for 4-byte keys).
 //
 // Every pass is stable and ties keep their row order, so the result is
 // exactly the stable order over all keys.  A one-key chunk with a run longer
@@ -193,20 +193,24 @@ __global__ void __launch_bounds__(256) k_msd_chunks(MsdChunkArgs a) {
 // ---------------------------------------------------------------------------
 // 5. shared-memory finish, one CTA per chunk
 // ---------------------------------------------------------------------------
+// Shared memory of a chunk of CAP rows: keys | row ids | bins (or the LSD
+// passes' per-warp counters) | chunk positions | small words.  The key-1
+// images of tied rows take the row ids' and bins' place: they are needed
+// only between the last use of the bins and the row ids' exchange.
 template <typename K, int THREADS, int ITEMS>
 struct LocalCfg {
     static constexpr int WARPS = THREADS / 32;
     static constexpr int CAP = THREADS * ITEMS;
+    static constexpr int NB = CAP;                  // counting bins: one per row a chunk can hold
+    static constexpr int BPT = NB / THREADS;        // bins per thread of the scan
     static constexpr size_t KEYS = (size_t)CAP * sizeof(K);
     static constexpr size_t VALS = (size_t)CAP * 4;
-    static constexpr size_t SEC = (size_t)CAP * 8;  // key 1 images of rows in runs; the counting pass's bins
+    static constexpr size_t BINS = (size_t)NB * 4 > (size_t)WARPS * 256 * 4 ? (size_t)NB * 4 : (size_t)WARPS * 256 * 4;
+    static constexpr size_t ORIG = (size_t)CAP * 2;  // chunk position of each slot's row; the dense-index table
     static constexpr size_t MISC = 16 * 4 + (size_t)WARPS * 4 + (size_t)2 * WARPS * 8;
-    static constexpr size_t ORIG = (size_t)CAP * 2;  // chunk position of each slot's row
-    static constexpr size_t SBIN = (size_t)CAP * 2;  // bin of each slot's row
-    static constexpr size_t SMEM = KEYS + VALS + SEC + MISC + ORIG + SBIN;
-    // the counting pass's 8192 bins and the LSD passes' per-warp counters
-    // live in the key-1 buffer, which is only needed after either is done
-    static_assert(SEC >= (size_t)2 * CAP * 4 && SEC >= (size_t)WARPS * 256 * 4, "key-1 buffer doubles as counters");
+    static constexpr size_t SMEM = KEYS + VALS + BINS + ORIG + MISC;
+    static_assert(VALS + BINS >= (size_t)CAP * 8 && (KEYS % 16) == 0 && (VALS % 16) == 0, "key-1 images");
+    static_assert(BPT % 4 == 0 && ORIG >= (size_t)NB * 2, "bin layout");
 };
 
 template <int THREADS>
@@ -221,14 +225,11 @@ __device__ __forceinline__ uint32_t local_excl_scan(uint32_t v, uint32_t* wsum, 
     }
     if (lane == 31) wsum[warp] = incl;
     __syncthreads();
-    uint32_t base = 0, all = 0;
-#pragma unroll
-    for (int w = 0; w < WARPS; ++w) {
-        const uint32_t x = wsum[w];
-        base += (w < warp) ? x : 0u;
-        all += x;
-    }
-    *total = all;
+    // every warp sums the earlier warps' totals with one reduction
+    static_assert(WARPS <= 32, "one lane per warp total");
+    const uint32_t t = lane < WARPS ? wsum[lane] : 0u;
+    const uint32_t base = __reduce_add_sync(0xffffffffu, lane < warp ? t : 0u);
+    *total = __reduce_add_sync(0xffffffffu, t);
     return base + incl - v;
 }
 
@@ -321,17 +322,6 @@ __device__ __forceinline__ void local_pass(K (&key)[ITEMS], uint32_t (&val)[ITEM
     }
 }
 
-// The chunk's rows in one counting pass: bin = (key - min) >> S with S the
-// smallest shift that brings the chunk's key range below 8192 bins, so rows
-// of spread keys fall about one per bin or fewer.  Rows land in their bin in no
-// particular order (shared-memory atomics); then each run of rows sharing a
-// bin is ranked by (key, key 1's order image, position in the chunk) --
-// positions are the rows' stable order so far -- which restores the exact
-// stable order.  Returns false, with nothing written to global memory, when
-// some run is longer than kMsdRunMax (many equal or clustered keys): the
-// caller then sorts the chunk with LSD passes instead.  On success item j of
-// a thread holds the row of slot (warp * ia + j) * 32 + lane and its final
-// position in the chunk is newpos[j].
 // Warp-wide minimum / maximum with the 32-bit reduce instructions: 8-byte
 // keys reduce their high halves first, then the low halves of the lanes that
 // hold the extreme high half.
@@ -348,108 +338,189 @@ __device__ __forceinline__ uint64_t warp_max(uint64_t x) {
     return ((uint64_t)hi << 32) | lo;
 }
 
-template <typename K, int THREADS, int ITEMS, int MATCH>
-__device__ __forceinline__ bool counting_finish(K (&key)[ITEMS], uint32_t (&val)[ITEMS], uint32_t (&newpos)[ITEMS],
-                                                uint32_t m, uint32_t ia, const MsdLocalArgs& a, K* sk, uint32_t* sv,
-                                                uint16_t* so, uint16_t* sbin, uint64_t* ssec, uint32_t* misc,
-                                                uint32_t* wsum, K* wmin, K* wmax) {
-    // the bins live in the key-1 buffer, which is not needed before the
-    // scatter is done
-    uint32_t* bins = reinterpret_cast<uint32_t*>(ssec);
-    constexpr int WARPS = THREADS / 32;
-    // bins (two per slot: 8192 for 4096-row chunks), bins per thread
-    constexpr int NB = 2 * THREADS * ITEMS, BPT = NB / THREADS;
-    constexpr int LNB = NB == 16384 ? 14 : 13;
-    static_assert((1 << LNB) == NB && BPT % 4 == 0, "bin layout");
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // ---- key range of the chunk
-    K kmin = ~K(0), kmax = 0;
-#pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-        const uint32_t pos = ((uint32_t)warp * ia + j) * 32 + lane;
-        if (j < (int)ia && pos < m) {
-            kmin = min(kmin, key[j]);
-            kmax = max(kmax, key[j]);
+// 1 when (key ak, position ao) comes before (bk, bo): the borrow of one
+// multi-word subtraction, four instructions with no branch.
+__device__ __forceinline__ uint32_t row_less(uint64_t ak, uint32_t ao, uint64_t bk, uint32_t bo) {
+    uint32_t r;
+    asm("{\n .reg .u32 t;\n sub.cc.u32 t, %1, %2;\n subc.cc.u32 t, %3, %4;\n subc.cc.u32 t, %5, %6;\n"
+        " subc.u32 %0, 0, 0;\n}"
+        : "=r"(r)
+        : "r"(ao), "r"(bo), "r"((uint32_t)ak), "r"((uint32_t)bk), "r"((uint32_t)(ak >> 32)), "r"((uint32_t)(bk >> 32)));
+    return 0u - r;
+}
+__device__ __forceinline__ uint32_t row_less(uint32_t ak, uint32_t ao, uint32_t bk, uint32_t bo) {
+    uint32_t r;
+    asm("{\n .reg .u32 t;\n sub.cc.u32 t, %1, %2;\n subc.cc.u32 t, %3, %4;\n subc.u32 %0, 0, 0;\n}"
+        : "=r"(r)
+        : "r"(ao), "r"(bo), "r"(ak), "r"(bk));
+    return 0u - r;
+}
+
+// A monotone map of the keys in [lo, hi] to bins [0, NB): a 32-bit window of
+// key - lo (all of it when the range fits), scaled by NB / range with one
+// high multiply, so that spread keys fill all NB bins evenly whatever the
+// range.  The scale is rounded down by more than its float error, so the
+// largest window stays below NB.
+template <typename K, int NB>
+struct BinMap {
+    K lo, hi;
+    uint32_t sh, mult;
+    bool direct;  // fewer than NB windows: the window is the bin
+    __device__ __forceinline__ void set(K l, K h) {
+        lo = l;
+        hi = h;
+        const K range = h - l;
+        uint32_t rw;
+        if constexpr (sizeof(K) == 8) {
+            const uint32_t top = (uint32_t)(range >> 32);
+            sh = top ? 32u - __clz((int)top) : 0u;
+            rw = __funnelshift_rc((uint32_t)range, top, sh);
+        } else {
+            sh = 0;
+            rw = range;
         }
+        direct = rw < (uint32_t)NB;
+        mult = direct ? 0u : (uint32_t)__fdividef((float)NB * 4294967296.0f * 0.999999f, (float)rw + 1.0f);
     }
-    kmin = warp_min(kmin);
-    kmax = warp_max(kmax);
-    if (lane == 0) {
-        wmin[warp] = kmin;
-        wmax[warp] = kmax;
+    __device__ __forceinline__ uint32_t operator()(K k) const {
+        const K off = k - lo;
+        uint32_t w;
+        if constexpr (sizeof(K) == 8) w = __funnelshift_rc((uint32_t)off, (uint32_t)(off >> 32), sh);
+        else w = off;
+        // the clamp never acts on keys in [lo, hi]; it keeps the bins in
+        // bounds for the rows a timed-out look-back left out of place
+        return min(direct ? w : __umulhi(w, mult), (uint32_t)NB - 1u);
     }
+};
+
+// The chunk's rows in one counting pass over NB bins of the chunk's key
+// range (BinMap; the range is the chunk's first and last bucket, known from
+// the rows' order, so no reduction over the keys is needed).  The histogram's
+// atomics also hand every row its arrival index in its bin; after the scan a
+// row alone in its bin is in its final position, and the few rows sharing a
+// bin are ranked among themselves by (key, key 1's order image, position in
+// the chunk) -- positions are the rows' stable order so far --, which
+// restores the exact stable order.  Where a bin holds more than kMsdRunMax
+// rows, the bins are laid out again over the keys' own range if that is less
+// than half as wide (clustered keys), else (many equal keys) stable passes
+// over the dense bin index order the rows.  On success the rows are in sk /
+// sv by final position; false (nothing written to global memory): the caller
+// sorts the chunk with LSD passes.
+template <typename K, int THREADS, int ITEMS, int MATCH>
+__device__ __forceinline__ bool counting_finish(K (&key)[ITEMS], uint32_t (&val)[ITEMS], uint32_t m, uint32_t ia,
+                                                K lo, K hi, const MsdLocalArgs& a, K* sk, uint32_t* sv, uint16_t* so,
+                                                uint32_t* bins, uint64_t* ssec, uint32_t* wsum, K* wmin, K* wmax) {
+    using C = LocalCfg<K, THREADS, ITEMS>;
+    constexpr int WARPS = C::WARPS, NB = C::NB, BPT = C::BPT;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t pos0 = (uint32_t)warp * ia * 32 + lane;  // item j's position: pos0 + 32 j
+    BinMap<K, NB> bin;
+    bin.set(lo, hi);
+    uint32_t br[ITEMS];  // bin | arrival index in the bin << 16
+    uint32_t cnt[BPT], tsum;
+    bool narrowed = false;
+#pragma unroll 1
+    for (;;) {  // at most twice; the bins are clear
 #pragma unroll
-    for (int i = 0; i < BPT; i += 4) *reinterpret_cast<uint4*>(bins + tid * BPT + i) = make_uint4(0, 0, 0, 0);
-    __syncthreads();
-    kmin = warp_min(lane < WARPS ? wmin[lane] : ~K(0));
-    kmax = warp_max(lane < WARPS ? wmax[lane] : K(0));
-    const K range = kmax - kmin;
-    int bl = 0;  // bit length of the range
-    if constexpr (sizeof(K) == 8) bl = range ? 64 - __clzll((long long)range) : 0;
-    else bl = range ? 32 - __clz((int)range) : 0;
-    const uint32_t S = bl > 13 ? (uint32_t)(bl - 13) : 0u;
-    auto bin_of = [&](K k) -> uint32_t { return (uint32_t)((k - kmin) >> S); };
-    // ---- histogram, exclusive scan, scatter
+        for (int j = 0; j < ITEMS; ++j) {
+            br[j] = 0;
+            if (j < (int)ia && pos0 + 32 * j < m) {
+                const uint32_t b = bin(key[j]);
+                br[j] = b | (atomicAdd(&bins[b], 1u) << 16);
+            }
+        }
+        __syncthreads();
+        uint32_t tmax = 0;
+        tsum = 0;
 #pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-        const uint32_t pos = ((uint32_t)warp * ia + j) * 32 + lane;
-        if (j < (int)ia && pos < m) atomicAdd(&bins[bin_of(key[j])], 1u);
-    }
-    __syncthreads();
-    // one scan of packed words: rows before the bin (low 16 bits) and
-    // occupied bins before it (high 16 bits: the bin's dense index)
-    uint32_t b[BPT];
-    uint32_t tsum = 0, tmax = 0;
+        for (int i = 0; i < BPT; i += 4) {
+            const uint4 q = *reinterpret_cast<const uint4*>(bins + tid * BPT + i);
+            cnt[i] = q.x;
+            cnt[i + 1] = q.y;
+            cnt[i + 2] = q.z;
+            cnt[i + 3] = q.w;
+        }
 #pragma unroll
-    for (int i = 0; i < BPT; i += 4) {
-        const uint4 q = *reinterpret_cast<const uint4*>(bins + tid * BPT + i);
-        b[i] = q.x;
-        b[i + 1] = q.y;
-        b[i + 2] = q.z;
-        b[i + 3] = q.w;
-    }
+        for (int i = 0; i < BPT; ++i) {
+            tmax = max(tmax, cnt[i]);
+            tsum += cnt[i];
+        }
+        if (__syncthreads_or(tmax > kMsdRunMax) == 0) break;
+        // A bin holds more rows than the direct ranking takes (many equal or
+        // clustered keys).
+        uint32_t occ = 0, total, b0 = NB, b1 = 0;  // occupied bins: how many, the first and last
 #pragma unroll
-    for (int i = 0; i < BPT; ++i) {
-        const uint32_t c = b[i];
-        tmax = max(tmax, c);
-        b[i] = tsum;
-        tsum += c + (c ? (1u << 16) : 0u);
-    }
-    uint32_t all;
-    const uint32_t start = local_excl_scan<THREADS>(tsum, wsum, &all);
-    if (__syncthreads_or(tmax > kMsdRunMax)) {
-        // A bin holds a run longer than the direct ranking takes (many equal
-        // or clustered keys): stable passes over the dense bin index instead
-        // of the scatter -- one when at most 256 bins are occupied, else two
-        // -- keep each bin's rows in their stable order, which is the final
-        // order wherever a bin holds one key value.  The dense index table
-        // takes the position and bin buffers (unused on this path).
-        static_assert(2 * (size_t)THREADS * ITEMS >= NB, "dense table fits the position and bin buffers");
-        uint16_t* dt = so;
+        for (int i = 0; i < BPT; ++i) {
+            if (cnt[i]) {
+                ++occ;
+                b0 = min(b0, (uint32_t)(tid * BPT + i));
+                b1 = tid * BPT + i;
+            }
+        }
+        b0 = __reduce_min_sync(0xffffffffu, b0);
+        b1 = __reduce_max_sync(0xffffffffu, b1);
+        if (lane == 0) wmin[warp] = (K)((b1 << 16) | b0);
+        uint32_t dn = local_excl_scan<THREADS>(occ, wsum, &total);
+        b0 = lane < WARPS ? (uint32_t)wmin[lane] & 0xffffu : (uint32_t)NB;
+        b1 = lane < WARPS ? (uint32_t)wmin[lane] >> 16 : 0u;
+        b0 = __reduce_min_sync(0xffffffffu, b0);
+        b1 = __reduce_max_sync(0xffffffffu, b1);
+        if (!narrowed && b1 - b0 < NB / 2) {  // uniform over the CTA
+            // the rows sit in less than half of the range: the bins again,
+            // over the keys' own range
+            narrowed = true;
+            K kmin = ~K(0), kmax = 0;
 #pragma unroll
-        for (int i = 0; i < BPT; ++i) dt[tid * BPT + i] = (uint16_t)((start + b[i]) >> 16);
+            for (int j = 0; j < ITEMS; ++j) {
+                if (j < (int)ia && pos0 + 32 * j < m) {
+                    kmin = min(kmin, key[j]);
+                    kmax = max(kmax, key[j]);
+                }
+            }
+            kmin = warp_min(kmin);
+            kmax = warp_max(kmax);
+            __syncthreads();  // wmin has been read
+            if (lane == 0) {
+                wmin[warp] = kmin;
+                wmax[warp] = kmax;
+            }
+#pragma unroll
+            for (int i = 0; i < BPT; i += 4)
+                *reinterpret_cast<uint4*>(bins + tid * BPT + i) = make_uint4(0, 0, 0, 0);
+            __syncthreads();
+            kmin = warp_min(lane < WARPS ? wmin[lane] : ~K(0));
+            kmax = warp_max(lane < WARPS ? wmax[lane] : K(0));
+            bin.set(kmin, kmax);
+            __syncthreads();  // ... and again, before it may be written again
+            continue;
+        }
+        // Stable passes over the dense bin index -- one when at most 256 bins
+        // are occupied, else two -- keep each bin's rows in their stable
+        // order, which is the final order wherever a bin holds one key value.
+        uint16_t* dt = so;  // dense index of each bin
+#pragma unroll
+        for (int i = 0; i < BPT; ++i) {
+            dt[tid * BPT + i] = (uint16_t)dn;
+            dn += cnt[i] ? 1u : 0u;
+        }
         __syncthreads();
         // slots past the chunk (all-ones keys) take the largest index, so they stay last
-        auto dense = [&](K k) -> uint32_t {
-            const K off = (k - kmin) >> S;
-            return off < (K)NB ? (uint32_t)dt[(uint32_t)off] : 0xffffu;
-        };
-        uint32_t* wcnt = bins;  // the bin counts are no longer needed
-        if ((all >> 16) <= 256) {
+        auto dense = [&](K k) -> uint32_t { return k > bin.hi ? 0xffffu : (uint32_t)dt[bin(k)]; };
+        if (total <= 256) {
             local_pass<K, THREADS, ITEMS, MATCH>(
-                key, val, [&](K k) { return min(dense(k), 255u); }, ia, sk, sv, wcnt, wsum, a.err);
+                key, val, [&](K k) { return min(dense(k), 255u); }, ia, sk, sv, bins, wsum, a.err);
         } else {
             local_pass<K, THREADS, ITEMS, MATCH>(
-                key, val, [&](K k) { return dense(k) & 0xffu; }, ia, sk, sv, wcnt, wsum, a.err);
+                key, val, [&](K k) { return dense(k) & 0xffu; }, ia, sk, sv, bins, wsum, a.err);
             local_pass<K, THREADS, ITEMS, MATCH>(
-                key, val, [&](K k) { return dense(k) >> 8; }, ia, sk, sv, wcnt, wsum, a.err);
+                key, val, [&](K k) { return dense(k) >> 8; }, ia, sk, sv, bins, wsum, a.err);
         }
         // in order now unless some bin holds several key values (or, with a
         // second key, key 0 ties): then the caller's LSD passes take over
         bool bad = false;
 #pragma unroll
         for (int j = 0; j < ITEMS; ++j) {
-            const uint32_t pos = ((uint32_t)warp * ia + j) * 32 + lane;
+            const uint32_t pos = pos0 + 32 * j;
             if (j < (int)ia && pos > 0 && pos < m) {
                 const K prev = sk[pos - 1];
                 bad |= a.sec ? !(prev < key[j]) : (prev > key[j]);
@@ -457,126 +528,145 @@ __device__ __forceinline__ bool counting_finish(K (&key)[ITEMS], uint32_t (&val)
         }
         return __syncthreads_or(bad) == 0;
     }
+    // ---- bin starts (with the count, one word per bin), rows into their slots
+    uint32_t all;
+    uint32_t run = local_excl_scan<THREADS>(tsum, wsum, &all);
 #pragma unroll
-    for (int i = 0; i < BPT; i += 4)
-        *reinterpret_cast<uint4*>(bins + tid * BPT + i) =
-            make_uint4((start + b[i]) & 0xffffu, (start + b[i + 1]) & 0xffffu, (start + b[i + 2]) & 0xffffu,
-                       (start + b[i + 3]) & 0xffffu);
+    for (int i = 0; i < BPT; i += 4) {
+        uint4 q;
+        q.x = run | (cnt[i] << 16);
+        run += cnt[i];
+        q.y = run | (cnt[i + 1] << 16);
+        run += cnt[i + 1];
+        q.z = run | (cnt[i + 2] << 16);
+        run += cnt[i + 2];
+        q.w = run | (cnt[i + 3] << 16);
+        run += cnt[i + 3];
+        *reinterpret_cast<uint4*>(bins + tid * BPT + i) = q;
+    }
     __syncthreads();
+    uint32_t fin[ITEMS];  // slot | rows in the bin << 16 (0: alone), then final position | moved << 16
 #pragma unroll
     for (int j = 0; j < ITEMS; ++j) {
-        const uint32_t pos = ((uint32_t)warp * ia + j) * 32 + lane;
-        if (j < (int)ia && pos < m) {
-            const uint32_t bn = bin_of(key[j]);
-            uint32_t slot = atomicAdd(&bins[bn], 1u);
+        fin[j] = 0;
+        if (j < (int)ia && pos0 + 32 * j < m) {
+            const uint32_t w = bins[br[j] & 0xffffu];
+            uint32_t slot = (w & 0xffffu) + (br[j] >> 16);
             if (slot >= m) {  // never when the counts are consistent
                 atomicOr(a.err, ERR_BAD_INDEX);
-                slot = pos;
+                slot = pos0 + 32 * j;
             }
+            const bool shared = (w >> 16) > 1;
+            fin[j] = shared ? slot | (w & 0xffff0000u) : slot;
             sk[slot] = key[j];
-            sv[slot] = val[j];
-            so[slot] = (uint16_t)pos;
-            sbin[slot] = (uint16_t)bn;
+            if (shared) so[slot] = (uint16_t)(pos0 + 32 * j);
+            br[j] = w & 0xffffu;  // the bin's first slot
         }
     }
     __syncthreads();
-    // ---- rows by slot; runs of one bin (bounds from ballots over each
-    //      32-slot group, loops only for runs that cross a group), and key 1
-    //      where key 0 ties inside a run
-    uint32_t run[ITEMS];  // s | e << 16; 0: alone in its bin
-    const uint32_t lt = lanemask_lt();
+    // ---- rows sharing a bin: each looks at the bin's slots
+    bool ties = false;  // some row's key 0 ties (two keys): key 1 decides
 #pragma unroll
     for (int j = 0; j < ITEMS; ++j) {
-        const uint32_t base = ((uint32_t)warp * ia + j) * 32;
-        const uint32_t p = base + lane;
-        newpos[j] = p;
-        run[j] = 0;
-        if (j < (int)ia) {
-            bool first = true, last = true;
-            uint32_t h = 0;
-            if (p < m) {
-                key[j] = sk[p];
-                val[j] = sv[p];
-                h = sbin[p];
-                first = p == 0 || sbin[p - 1] != h;
-                last = p + 1 >= m || sbin[p + 1] != h;
-            }
-            const uint32_t starts = __ballot_sync(0xffffffffu, first);
-            const uint32_t ends = __ballot_sync(0xffffffffu, last);
-            if (!(first && last)) {
-                const uint32_t sm = starts & (lt | (1u << lane));  // starts at lanes <= this one
-                const uint32_t em = ends & ~lt;                    // ends at lanes >= this one
-                uint32_t s = sm ? base + 31 - __clz(sm) : base;
-                uint32_t e = em ? base + __ffs(em) : base + 32;
-                if (!sm)
-                    while (s > 0 && p - s < kMsdRunMax && sbin[s - 1] == h) --s;
-                if (!em)
-                    while (e < m && e - p <= kMsdRunMax && sbin[e] == h) ++e;
-                run[j] = s | (e << 16);
-                if (e - s > kMsdRunMax) {
-                    misc[4] = 1;
-                } else if (a.sec) {
-                    bool tie = false;
-                    for (uint32_t t = s; t < e; ++t) tie |= (t != p) && sk[t] == key[j];
-                    if (tie) {
-                        uint32_t row = val[j];
-                        if (row >= a.n) {  // never for a permutation of [0, n)
-                            atomicOr(a.err, ERR_BAD_INDEX);
-                            row = 0;
-                        }
-                        ssec[p] = sec_image(a.sec, a.sec_dtype, row, a.invert != 0);
-                    }
-                }
-            }
-        }
-    }
-    __syncthreads();
-    if (misc[4]) return false;
-#pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-        if (run[j] == 0) continue;
-        const uint32_t p = ((uint32_t)warp * ia + j) * 32 + lane;
-        const uint32_t s = run[j] & 0xffffu, e = run[j] >> 16;
+        const uint32_t c = fin[j] >> 16;
+        if (c <= 1) continue;
+        const uint32_t slot = fin[j] & 0xffffu, end = br[j] + c;
         const K k = key[j];
-        const uint32_t o = so[p];
-        uint32_t r = 0;
-        for (uint32_t t = s; t < e; ++t) {
-            const K tk = sk[t];
-            bool less = tk < k;
-            if (tk == k && t != p) {
-                const uint32_t to = so[t];
-                if (a.sec) {
-                    const uint64_t sc = ssec[p], tsc = ssec[t];
-                    less = tsc < sc || (tsc == sc && to < o);
-                } else {
-                    less = to < o;
-                }
+        uint32_t r = br[j];
+        bool tie = false;
+        if (a.sec) {
+            uint32_t t = slot;
+#pragma unroll 1
+            for (uint32_t i = 1; i < c; ++i) {
+                if (++t == end) t = br[j];
+                const K tk = sk[t];
+                tie |= tk == k;
+                r += tk < k ? 1u : 0u;
             }
-            r += less ? 1u : 0u;
+        } else {
+            const uint32_t o = pos0 + 32 * j;
+#pragma unroll 1
+            for (uint32_t t = br[j]; t < end; ++t) r += row_less(sk[t], so[t], k, o);
         }
-        newpos[j] = s + r;
+        if (tie) {
+            ties = true;
+            uint32_t row = val[j];
+            if (row >= a.n) {  // never for a permutation of [0, n)
+                atomicOr(a.err, ERR_BAD_INDEX);
+                row = 0;
+            }
+            ssec[slot] = sec_image(a.sec, a.sec_dtype, row, a.invert != 0);
+            br[j] |= 0x10000u;  // ranked again below
+        } else {
+            fin[j] = r | (r != slot ? 0x10000u : 0u);  // bit 16: the row moves
+        }
     }
+    if (a.sec && __syncthreads_or(ties)) {
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) {
+            if (!(br[j] >> 16)) continue;
+            const uint32_t b0 = br[j] & 0xffffu;
+            const uint32_t c = fin[j] >> 16, slot = fin[j] & 0xffffu, end = b0 + c;
+            const K k = key[j];
+            const uint64_t sc = ssec[slot];
+            uint32_t r = b0, t = slot;
+#pragma unroll 1
+            for (uint32_t i = 1; i < c; ++i) {
+                if (++t == end) t = b0;
+                const K tk = sk[t];
+                bool less = tk < k;
+                if (tk == k) {
+                    const uint64_t tsc = ssec[t];
+                    less = tsc < sc || (tsc == sc && so[t] < pos0 + 32 * j);
+                }
+                r += less ? 1u : 0u;
+            }
+            fin[j] = r | (r != slot ? 0x10000u : 0u);
+        }
+    }
+    __syncthreads();  // every slot has been compared: rows to their final positions
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+        if (j < (int)ia && pos0 + 32 * j < m) {
+            const uint32_t f = fin[j] & 0xffffu;
+            if (fin[j] >> 16) sk[f] = key[j];
+            sv[f] = val[j];
+        }
+    }
+    __syncthreads();
     return true;
 }
 
-// MATCH: 0 = one ballot per digit bit, 1 = match.any.
+// Issue-bound: what counts is instructions per row and the barriers between
+// the phases.  Hence one histogram atomic per row whose result is also the
+// row's slot (no second counting pass), bins scaled to the chunk's range
+// without a reduction over its keys, a bin per row of capacity (half full on
+// average: four rows in ten share one), ranking in registers with only the
+// shared rows' compares going through shared memory, and one branch-free
+// multi-word compare per slot.  100M rows of two keys, one B200: 2.80 ms
+// before (506 instructions per row: two atomic passes over 8,192 bins, rows
+// re-read by slot with their run bounds found by ballots), 1.33 ms now (247
+// per row, 57 % of issue slots); 200M rows of 50M keys in 8,192-row chunks
+// 7.1 -> 4.2 ms; 50M rows of 25M keys 1.40 -> 0.80 ms.  HBM would take the
+// 24 bytes per row in 0.37 ms per 100M rows.
+//
+// MATCH (the stable passes): 0 = one ballot per digit bit, 1 = match.any.
 template <typename K, int THREADS, int ITEMS, int MATCH>
-__global__ void __launch_bounds__(THREADS, THREADS >= 1024 ? 1 : 2) k_msd_local(MsdLocalArgs a) {
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_msd_local(MsdLocalArgs a) {
     using C = LocalCfg<K, THREADS, ITEMS>;
-    constexpr int WARPS = C::WARPS, RADIX = 256;
+    constexpr int WARPS = C::WARPS;
     constexpr uint32_t CAP = (uint32_t)C::CAP;
     constexpr int KBITS = 8 * (int)sizeof(K);
     extern __shared__ __align__(16) unsigned char smem[];
     K* sk = reinterpret_cast<K*>(smem);
     uint32_t* sv = reinterpret_cast<uint32_t*>(smem + C::KEYS);
-    uint64_t* ssec = reinterpret_cast<uint64_t*>(smem + C::KEYS + C::VALS);
-    uint32_t* wcnt = reinterpret_cast<uint32_t*>(ssec);                                 // [WARPS][RADIX]
-    uint32_t* misc = reinterpret_cast<uint32_t*>(smem + C::KEYS + C::VALS + C::SEC);  // [0], [4]: long runs
-    uint32_t* wsum = misc + 16;                                                       // [WARPS]
-    K* wor = reinterpret_cast<K*>(smem + C::KEYS + C::VALS + C::SEC + 16 * 4 + WARPS * 4);
+    uint64_t* ssec = reinterpret_cast<uint64_t*>(smem + C::KEYS);  // over the row ids and bins
+    uint32_t* wcnt = reinterpret_cast<uint32_t*>(smem + C::KEYS + C::VALS);  // bins, or [WARPS][RADIX]
+    uint16_t* so = reinterpret_cast<uint16_t*>(smem + C::KEYS + C::VALS + C::BINS);
+    uint32_t* misc = reinterpret_cast<uint32_t*>(smem + C::KEYS + C::VALS + C::BINS + C::ORIG);  // [0]: long runs
+    uint32_t* wsum = misc + 16;                                                                  // [WARPS]
+    K* wor = reinterpret_cast<K*>(smem + C::KEYS + C::VALS + C::BINS + C::ORIG + 16 * 4 + WARPS * 4);
     K* wand = wor + WARPS;
-    uint16_t* so = reinterpret_cast<uint16_t*>(smem + C::KEYS + C::VALS + C::SEC + C::MISC);
-    uint16_t* sbin = so + CAP;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // the flag a failing chunk raises: the sort's, or its segment's
@@ -588,14 +678,18 @@ __global__ void __launch_bounds__(THREADS, THREADS >= 1024 ? 1 : 2) k_msd_local(
         misc[1] = *static_cast<volatile uint32_t*>(fail_word);
         misc[2] = a.chunk_start[blockIdx.x];
         uint32_t e = a.chunk_start[blockIdx.x + 1];
-        if (a.seg_chunks) e = min(e, a.seg_chunks[blockIdx.x].seg_end);  // the segment's last chunk
+        uint32_t ps = a.pshift;
+        if (a.seg_chunks) {
+            e = min(e, a.seg_chunks[blockIdx.x].seg_end);  // the segment's last chunk
+            ps = a.seg_chunks[blockIdx.x].pshift;
+        }
         misc[3] = e;
+        misc[4] = ps;
         misc[0] = 0;
-        misc[4] = 0;
     }
     __syncthreads();
     if (misc[1]) return;  // the plan failed earlier: the LSD passes take over
-    const uint32_t s0 = misc[2], s1 = misc[3];
+    const uint32_t s0 = misc[2], s1 = misc[3], pshift = misc[4];
     if (s1 <= s0) return;
     const uint32_t m = s1 - s0;
     if (m > CAP || s1 > a.n) {
@@ -603,6 +697,8 @@ __global__ void __launch_bounds__(THREADS, THREADS >= 1024 ? 1 : 2) k_msd_local(
         return;
     }
     const uint32_t ia = (m + THREADS - 1) / THREADS;  // items per thread in use
+#pragma unroll
+    for (int i = 0; i < C::BPT; i += 4) *reinterpret_cast<uint4*>(wcnt + tid * C::BPT + i) = make_uint4(0, 0, 0, 0);
 
     // ---- load: item j of a thread sits at position (warp * ia + j) * 32 + lane;
     //      slots past m hold all-ones keys, which every pass ranks last
@@ -610,9 +706,10 @@ __global__ void __launch_bounds__(THREADS, THREADS >= 1024 ? 1 : 2) k_msd_local(
     uint32_t val[ITEMS];
     const K* kin = static_cast<const K*>(a.keys) + s0;
     const uint32_t* vin = a.vals + s0;
+    const uint32_t pos0 = (uint32_t)warp * ia * 32 + lane;
 #pragma unroll
     for (int j = 0; j < ITEMS; ++j) {
-        const uint32_t pos = ((uint32_t)warp * ia + j) * 32 + lane;
+        const uint32_t pos = pos0 + 32 * j;
         key[j] = ~K(0);
         val[j] = 0;
         if (j < (int)ia && pos < m) {
@@ -620,30 +717,61 @@ __global__ void __launch_bounds__(THREADS, THREADS >= 1024 ? 1 : 2) k_msd_local(
             val[j] = ldg_stream(vin + pos);
         }
     }
+    K carry = 0;  // the row before this warp's
+    if (pos0 - lane > 0 && pos0 - lane < m) carry = kin[pos0 - lane - 1];
+    const K first = kin[0], last = kin[m - 1];
 
     // ---- rows already in order (with one key: non-decreasing; with two:
     //      increasing, so key 1 decides nothing) stay where they are; this is
     //      the common case when each bucket holds one key value
+    // (each warp's first 32 rows tell most chunks apart before the rest is looked at)
     bool in_order = true;
+    auto check = [&](int j) {
+        const uint32_t pos = pos0 + 32 * j;
+        const K before = __shfl_sync(0xffffffffu, key[j], (lane + 31) & 31);
+        const K prev = lane ? before : carry;
+        carry = before;  // lane 0: lane 31's key, the row before the next item's
+        if (pos > 0 && pos < m) in_order = in_order && (a.sec ? prev < key[j] : prev <= key[j]);
+    };
+    check(0);
+    bool ordered = __syncthreads_or(!in_order) == 0;
+    if (ordered && ia > 1) {
 #pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-        const uint32_t pos = ((uint32_t)warp * ia + j) * 32 + lane;
-        if (j < (int)ia) {
-            K prev = __shfl_up_sync(0xffffffffu, key[j], 1);
-            if (lane == 0 && pos > 0 && pos < m) prev = kin[pos - 1];
-            if (pos > 0 && pos < m) in_order = in_order && (a.sec ? prev < key[j] : prev <= key[j]);
-        }
+        for (int j = 1; j < ITEMS; ++j)
+            if (j < (int)ia) check(j);
+        ordered = __syncthreads_or(!in_order) == 0;
     }
-    in_order = __syncthreads_and(in_order) != 0;
-    uint32_t newpos[ITEMS];
+    K* kout = static_cast<K*>(a.keys_out);
+    if (ordered) {
 #pragma unroll
-    for (int j = 0; j < ITEMS; ++j) newpos[j] = ((uint32_t)warp * ia + j) * 32 + lane;
+        for (int j = 0; j < ITEMS; ++j) {
+            const uint32_t pos = pos0 + 32 * j;
+            if (j < (int)ia && pos < m) {
+                uint64_t gp = (uint64_t)s0 + pos;
+                if (a.reverse) gp = a.n - 1 - gp;
+                stg_stream(a.perm_out + gp, val[j]);
+                if (kout) stg_stream(kout + gp, KeyOps<K>::unorder(key[j], a.dtype, a.invert != 0));
+            }
+        }
+        return;
+    }
 
-    // ---- one counting pass over the chunk's key range; where that leaves a
+    // ---- one counting pass over the chunk's key range (whole buckets, so
+    //      the first and last row's top bits bound it); where that leaves a
     //      long run (many equal or clustered keys), stable LSD passes instead
-    const bool counted = in_order || counting_finish<K, THREADS, ITEMS, MATCH>(key, val, newpos, m, ia, a, sk, sv, so,
-                                                                               sbin, ssec, misc, wsum, wor, wand);
-    if (!counted) {
+    const K below = pshift < (uint32_t)KBITS ? (K)((((K)1) << pshift) - 1) : ~K(0);
+    if (counting_finish<K, THREADS, ITEMS, MATCH>(key, val, m, ia, first & ~below, last | below, a, sk, sv, so, wcnt,
+                                                  ssec, wsum, wor, wand)) {
+        for (uint32_t i = tid; i < m; i += THREADS) {
+            uint64_t gp = (uint64_t)s0 + i;
+            if (a.reverse) gp = a.n - 1 - gp;
+            stg_stream(a.perm_out + gp, sv[i]);
+            if (kout) stg_stream(kout + gp, KeyOps<K>::unorder(sk[i], a.dtype, a.invert != 0));
+        }
+        return;
+    }
+    uint32_t newpos[ITEMS];
+    {
         __syncthreads();
 #pragma unroll
         for (int j = 0; j < ITEMS; ++j) {
@@ -705,6 +833,8 @@ __global__ void __launch_bounds__(THREADS, THREADS >= 1024 ? 1 : 2) k_msd_local(
             }
             __syncthreads();
         }
+
+        __syncthreads();  // the row ids' buffer has been read back: key 1's images go over it
 
         // ---- runs of equal high bits, ranked by (low bits, key 1, position).
         //      Key 1 is read (through the row id) only for rows whose low bits
@@ -805,7 +935,6 @@ __global__ void __launch_bounds__(THREADS, THREADS >= 1024 ? 1 : 2) k_msd_local(
     }
 
     // ---- output: raw sorted key 0 and the permutation
-    K* kout = static_cast<K*>(a.keys_out);
 #pragma unroll
     for (int j = 0; j < ITEMS; ++j) {
         const uint32_t pos = ((uint32_t)warp * ia + j) * 32 + lane;
@@ -822,22 +951,38 @@ __global__ void __launch_bounds__(THREADS, THREADS >= 1024 ? 1 : 2) k_msd_local(
 // host side
 // ---------------------------------------------------------------------------
 namespace {
-constexpr int kLocalThreads = 512, kLocalItems = 8;
-static_assert(kLocalThreads * kLocalItems == (int)kMsdCap, "chunk capacity");
-static_assert(2 * kLocalThreads * kLocalItems == (int)kMsdWideCap, "wide chunk capacity");
+// Chunks of up to CAP rows, one CTA of CAP / 8 threads each: 4096 rows (two
+// CTAs per SM) or 8192 (one).
+constexpr int kLocalItems = 8;
 static_assert(kMsdWideCap < (1u << 16), "run bounds are packed in 16 bits");
-using Local64 = LocalCfg<uint64_t, kLocalThreads, kLocalItems>;
-using Local32 = LocalCfg<uint32_t, kLocalThreads, kLocalItems>;
-using Wide64 = LocalCfg<uint64_t, 2 * kLocalThreads, kLocalItems>;
-using Wide32 = LocalCfg<uint32_t, 2 * kLocalThreads, kLocalItems>;
-template <int MATCH>
-struct LocalKernels {
-    static constexpr auto k64 = k_msd_local<uint64_t, kLocalThreads, kLocalItems, MATCH>;
-    static constexpr auto k32 = k_msd_local<uint32_t, kLocalThreads, kLocalItems, MATCH>;
-    // wide chunks (<= 8192 rows): one CTA of 1024 threads per SM
-    static constexpr auto w64 = k_msd_local<uint64_t, 2 * kLocalThreads, kLocalItems, MATCH>;
-    static constexpr auto w32 = k_msd_local<uint32_t, 2 * kLocalThreads, kLocalItems, MATCH>;
+template <typename K, uint32_t CAP, int MATCH>
+struct Local {
+    static constexpr int THREADS = (int)CAP / kLocalItems;
+    static constexpr size_t SMEM = LocalCfg<K, THREADS, kLocalItems>::SMEM;
+    static cudaError_t prepare() {
+        return cudaFuncSetAttribute(k_msd_local<K, THREADS, kLocalItems, MATCH>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
+    }
+    static void launch(const MsdLocalArgs& a, uint32_t nchunks, cudaStream_t s) {
+        k_msd_local<K, THREADS, kLocalItems, MATCH><<<nchunks, THREADS, SMEM, s>>>(a);
+    }
 };
+template <typename K, uint32_t CAP>
+cudaError_t local_prepare() {
+    const cudaError_t e = Local<K, CAP, 0>::prepare();
+    return e == cudaSuccess ? Local<K, CAP, 1>::prepare() : e;
+}
+template <typename K, uint32_t CAP>
+void local_launch(const MsdLocalArgs& a, uint32_t nchunks, int match, cudaStream_t s) {
+    if (match) Local<K, CAP, 1>::launch(a, nchunks, s);
+    else Local<K, CAP, 0>::launch(a, nchunks, s);
+}
+template <typename K>
+void chunks_launch(const MsdChunkArgs& a, uint32_t cap, cudaStream_t s) {
+    const uint32_t grid = (a.nchunks + 1 + 7) / 8;
+    if (cap == kMsdWideCap) k_msd_chunks<K, kMsdWideCap><<<grid, 256, 0, s>>>(a);
+    else k_msd_chunks<K, kMsdCap><<<grid, 256, 0, s>>>(a);
+}
 
 int sm_count() {
     int dev = 0, sms = 148;
@@ -848,21 +993,11 @@ int sm_count() {
 }  // namespace
 
 cudaError_t prepare_msd_kernels() {
-    const void* k64[2] = {(const void*)LocalKernels<0>::k64, (const void*)LocalKernels<1>::k64};
-    const void* k32[2] = {(const void*)LocalKernels<0>::k32, (const void*)LocalKernels<1>::k32};
-    const void* w64[2] = {(const void*)LocalKernels<0>::w64, (const void*)LocalKernels<1>::w64};
-    const void* w32[2] = {(const void*)LocalKernels<0>::w32, (const void*)LocalKernels<1>::w32};
-    for (int m = 0; m < 2; ++m) {
-        cudaError_t e = cudaFuncSetAttribute(k64[m], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Local64::SMEM);
-        if (e != cudaSuccess) return e;
-        e = cudaFuncSetAttribute(k32[m], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Local32::SMEM);
-        if (e != cudaSuccess) return e;
-        e = cudaFuncSetAttribute(w64[m], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Wide64::SMEM);
-        if (e != cudaSuccess) return e;
-        e = cudaFuncSetAttribute(w32[m], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Wide32::SMEM);
-        if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
+    cudaError_t e = local_prepare<uint64_t, kMsdCap>();
+    if (e == cudaSuccess) e = local_prepare<uint64_t, kMsdWideCap>();
+    if (e == cudaSuccess) e = local_prepare<uint32_t, kMsdCap>();
+    if (e == cudaSuccess) e = local_prepare<uint32_t, kMsdWideCap>();
+    return e;
 }
 
 cudaError_t msd_hist(const MsdHistArgs& a, int width, cudaStream_t s) {
@@ -879,34 +1014,19 @@ cudaError_t msd_scan(const uint32_t* hist, uint32_t* offs, int ndig, uint32_t ca
 }
 
 cudaError_t msd_chunks(const MsdChunkArgs& a, int width, cudaStream_t s, uint32_t cap) {
-    const uint32_t grid = (a.nchunks + 1 + 7) / 8;
-    if (cap == kMsdWideCap) {
-        if (width == 8) k_msd_chunks<uint64_t, kMsdWideCap><<<grid, 256, 0, s>>>(a);
-        else k_msd_chunks<uint32_t, kMsdWideCap><<<grid, 256, 0, s>>>(a);
-    } else {
-        if (width == 8) k_msd_chunks<uint64_t, kMsdCap><<<grid, 256, 0, s>>>(a);
-        else k_msd_chunks<uint32_t, kMsdCap><<<grid, 256, 0, s>>>(a);
-    }
+    if (width == 8) chunks_launch<uint64_t>(a, cap, s);
+    else chunks_launch<uint32_t>(a, cap, s);
     return cudaGetLastError();
 }
 
 cudaError_t msd_local(const MsdLocalArgs& a, int width, uint32_t nchunks, int match, cudaStream_t s, uint32_t cap) {
     if (nchunks == 0) return cudaSuccess;
-    constexpr int WT = 2 * kLocalThreads;
     if (cap == kMsdWideCap) {
-        if (width == 8) {
-            if (match) LocalKernels<1>::w64<<<nchunks, WT, Wide64::SMEM, s>>>(a);
-            else LocalKernels<0>::w64<<<nchunks, WT, Wide64::SMEM, s>>>(a);
-        } else {
-            if (match) LocalKernels<1>::w32<<<nchunks, WT, Wide32::SMEM, s>>>(a);
-            else LocalKernels<0>::w32<<<nchunks, WT, Wide32::SMEM, s>>>(a);
-        }
-    } else if (width == 8) {
-        if (match) LocalKernels<1>::k64<<<nchunks, kLocalThreads, Local64::SMEM, s>>>(a);
-        else LocalKernels<0>::k64<<<nchunks, kLocalThreads, Local64::SMEM, s>>>(a);
+        if (width == 8) local_launch<uint64_t, kMsdWideCap>(a, nchunks, match, s);
+        else local_launch<uint32_t, kMsdWideCap>(a, nchunks, match, s);
     } else {
-        if (match) LocalKernels<1>::k32<<<nchunks, kLocalThreads, Local32::SMEM, s>>>(a);
-        else LocalKernels<0>::k32<<<nchunks, kLocalThreads, Local32::SMEM, s>>>(a);
+        if (width == 8) local_launch<uint64_t, kMsdCap>(a, nchunks, match, s);
+        else local_launch<uint32_t, kMsdCap>(a, nchunks, match, s);
     }
     return cudaGetLastError();
 }
