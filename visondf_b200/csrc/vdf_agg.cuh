@@ -5,6 +5,7 @@
 // and min/max in the column's order.
 #pragma once
 #include "vdf_common.cuh"
+#include "vdf_internal.h"
 
 namespace vdf {
 
@@ -65,6 +66,43 @@ __device__ __forceinline__ double i128_to_double(uint64_t lo, uint64_t hi, bool 
     }
     if (hi == 0) return (double)lo;
     return ldexp((double)hi, 64) + (double)lo;
+}
+
+
+__device__ __forceinline__ void store_raw(void* dst, int w, uint64_t i, uint64_t v) {
+    if (w == 4) static_cast<uint32_t*>(dst)[i] = (uint32_t)v;
+    else static_cast<unsigned long long*>(dst)[i] = v;
+}
+
+// Group g's record into the output columns.
+template <int NV>
+__device__ __forceinline__ void emit_group(const SegArgs& a, uint32_t g, uint32_t cnt, const uint64_t (*w)[4],
+                                           const int* vc) {
+    if (a.count_out) a.count_out[g] = (int64_t)cnt;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        const SegAggOut& o = a.agg[v];
+        const int dt = a.val[v].dtype;
+        if (vc[v] == VC_FLOAT) {
+            const double s = __dadd_rn(as_f(w[v][0]), as_f(w[v][1]));
+            if (o.sum) static_cast<double*>(o.sum)[g] = s;
+            if (o.mean) o.mean[g] = s / (double)cnt;
+            if (dt == F64) {
+                if (o.min) static_cast<double*>(o.min)[g] = as_f(w[v][2]);
+                if (o.max) static_cast<double*>(o.max)[g] = as_f(w[v][3]);
+            } else {
+                if (o.min) static_cast<float*>(o.min)[g] = (float)as_f(w[v][2]);
+                if (o.max) static_cast<float*>(o.max)[g] = (float)as_f(w[v][3]);
+            }
+        } else {
+            if (o.sum) static_cast<int64_t*>(o.sum)[g] = (int64_t)w[v][0];
+            if (o.sum_hi) o.sum_hi[g] = (int64_t)w[v][1];
+            if (o.mean) o.mean[g] = i128_to_double(w[v][0], w[v][1], vc[v] == VC_SINT) / (double)cnt;
+            const int wd = dtype_width(dt);
+            if (o.min) store_raw(o.min, wd, g, w[v][2]);
+            if (o.max) store_raw(o.max, wd, g, w[v][3]);
+        }
+    }
 }
 
 }  // namespace vdf

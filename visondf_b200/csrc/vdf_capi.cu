@@ -372,6 +372,7 @@ vdf_status vdf_ctx_create(int device, vdf_ctx** out) {
             e = vdf::prepare_sort_kernels();
             if (e == cudaSuccess) e = vdf::prepare_segreduce_kernels();
             if (e == cudaSuccess) e = vdf::prepare_batch_kernels();
+            if (e == cudaSuccess) e = vdf::prepare_dict_agg_kernels();
             if (e != cudaSuccess) {
                 delete c;
                 return VDF_ERR_DEVICE;
@@ -567,6 +568,75 @@ vdf_status vdf_groupby_sorted(vdf_ctx* c, uint64_t n, const vdf_col* keys, int n
 
 namespace {
 
+// Whether a call asks only for the group table of one key and synchronises
+// for the group count anyway, so that a group-by without a sort can be tried
+// (vdf_dictagg.cu), from the row count the dictionary plan of a sort is tried
+// at.
+bool wants_only_groups(vdf_ctx* c, const vdf_sort_groupby_args* x, cudaStream_t s) {
+    if (!x->groupby || x->nkeys != 1 || !x->n_groups_host || x->perm_in || x->perm_out || x->group_start_out ||
+        x->row_group_out)
+        return false;
+    if (x->sorted_keys_out && x->sorted_keys_out[0]) return false;
+    for (int p = 0; p < x->npayload; ++p)
+        if (x->payload_out && x->payload_out[p]) return false;
+    if (!c->tuning.dict || x->n < 2 || x->n < 4 * c->tuning.msd_min_rows) return false;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return false;
+    }
+    return true;
+}
+
+// The group-by without a sort: *done when the groups are written and counted;
+// else the key takes more than kDictMax values and the sorted path follows.
+// The values are first taken from a sample; when a row holds one that the
+// sample missed, they are collected from every row and the pass is repeated.
+vdf_status groups_without_sort(vdf_ctx* c, const vdf_sort_groupby_args* x, cudaStream_t s, bool* done) {
+    *done = false;
+    vdf_status st = ws_ensure(c, vdf::dict_agg_workspace_bytes());
+    if (st != VDF_OK) return st;
+    vdf::DictAggPlan p{};
+    p.order = x->order;
+    p.spin_limit = c->tuning.spin_limit;
+    p.taken = dict_word(c);
+    vdf::SegArgs& a = p.seg;
+    a.n = x->n;
+    a.nkeys = 1;
+    a.nvals = x->nagg;
+    a.key[0] = vdf::SegCol{x->keys[0].data, x->keys[0].dtype};
+    a.key_out[0] = x->group_keys_out ? x->group_keys_out[0] : nullptr;
+    for (int i = 0; i < x->nagg; ++i) {
+        const vdf_col& v = x->payload[x->agg_cols[i]];
+        a.val[i] = vdf::SegCol{v.data, v.dtype};
+        const vdf_agg_out& o = x->aggs[i];
+        a.agg[i] = vdf::SegAggOut{o.sum, o.sum_hi, o.min, o.max, o.mean};
+    }
+    a.count_out = x->group_count_out;
+    a.n_groups = x->n_groups_dev;
+    a.err = err_word(c);
+    c->dict_sorts++;
+    for (int sample = 1; sample >= 0; --sample) {
+        int launched = 0;
+        cudaError_t e = vdf::run_dict_agg(p, sample != 0, c->ws, s, prof_of(c), &launched);
+        c->launches += launched;
+        if (e != cudaSuccess) return from_cuda(c, e, "group-by of few keys");
+        static_assert(sizeof(vdf::DictAggWords) == 16, "two spare host words");
+        e = cudaMemcpyAsync(&c->host_pinned[6], c->ws, sizeof(vdf::DictAggWords), cudaMemcpyDeviceToHost, s);
+        if (e != cudaSuccess) return from_cuda(c, e, "read group words");
+        if ((st = drain_and_check(c, s)) != VDF_OK) return st;
+        vdf::DictAggWords w;
+        std::memcpy(&w, &c->host_pinned[6], sizeof w);
+        if (w.state == 2 && !w.missed) {
+            *x->n_groups_host = w.ndist;
+            *done = true;
+            return VDF_OK;
+        }
+        if (w.state != 2) return VDF_OK;  // too many values
+    }
+    return VDF_OK;
+}
+
 // vdf_sort_groupby with the context lock already held.
 vdf_status sort_groupby_locked(vdf_ctx* c, const vdf_sort_groupby_args* x, cudaStream_t stream) {
     vdf_status st;
@@ -602,7 +672,13 @@ vdf_status sort_groupby_locked(vdf_ctx* c, const vdf_sort_groupby_args* x, cudaS
         dts[k] = x->keys[k].dtype;
         cols[k] = x->keys[k].data;
     }
-    const vdf::SortPlan plan = vdf::make_sort_plan(n, dts, x->nkeys, c->tuning);
+    vdf::SortTuning tuning = c->tuning;
+    if (wants_only_groups(c, x, s)) {
+        bool done = false;
+        if ((st = groups_without_sort(c, x, s, &done)) != VDF_OK || done) return st;
+        tuning.dict = 0;  // the key takes too many values for the dictionary plan
+    }
+    const vdf::SortPlan plan = vdf::make_sort_plan(n, dts, x->nkeys, tuning);
     // Sorted copies needed by the group-by that the caller did not ask for
     // live in the workspace: [perm][key 0][keys 1..][aggregated payload][tail]
     // where tail = max(sort workspace, group-by workspace).

@@ -26,63 +26,11 @@
 #include <algorithm>
 
 #include "vdf_common.cuh"
+#include "vdf_dict.cuh"
 #include "vdf_internal.h"
 
 namespace vdf {
 namespace {
-
-__device__ __forceinline__ uint32_t ld_volatile(const uint32_t* p) { return *static_cast<const volatile uint32_t*>(p); }
-__device__ __forceinline__ unsigned long long ld_volatile(const unsigned long long* p) {
-    return *static_cast<const volatile unsigned long long*>(p);
-}
-
-// Adds `add` rows of value x to a CTA's open-addressing table in shared
-// memory (keys / counts / states).  A new value takes the next index of
-// *distinct; more than kDictMax of them, a full table or a wait that gives up
-// set *over.  Returns false when the value was not recorded.  The fences are
-// CTA-scoped: only the CTA's own threads read the table.
-__device__ bool dict_add(unsigned long long* keys, uint32_t* cnt, uint32_t* st, uint32_t mask, unsigned long long x,
-                         uint32_t add, uint32_t limit, uint32_t* distinct, uint32_t* over, uint32_t* err) {
-    uint32_t s = dict_hash(x) & mask;
-    for (uint32_t probe = 0; probe <= mask; ++probe) {
-        // too many values already: the table is not filled further.  Checked
-        // at every step, before a slot is claimed: with many distinct keys all
-        // the CTA's threads insert at once, and without it they would fill
-        // the table and probe it end to end after the plan has failed.
-        if (ld_volatile(over)) return false;
-        uint32_t state = ld_volatile(st + s);
-        if (state == 0) {
-            state = atomicCAS(st + s, 0u, 1u);
-            if (state == 0) {  // this thread owns the slot: key, then count, then publish
-                keys[s] = x;
-                atomicAdd(cnt + s, add);
-                __threadfence_block();
-                atomicExch(st + s, 2u);
-                if (atomicAdd(distinct, 1u) >= kDictMax) atomicOr(over, 1u);
-                return true;
-            }
-        }
-        uint32_t spins = 0;
-        while (state != 2) {  // another thread is writing the slot's key
-            if (ld_volatile(over)) return false;
-            if (++spins > limit) {
-                atomicOr(err, ERR_LOOKBACK_TIMEOUT);
-                atomicOr(over, 1u);
-                return false;
-            }
-            if (spins > 16) __nanosleep(32);
-            state = ld_volatile(st + s);
-        }
-        __threadfence_block();
-        if (ld_volatile(keys + s) == x) {
-            atomicAdd(cnt + s, add);
-            return true;
-        }
-        s = (s + 1) & mask;
-    }
-    atomicOr(over, 1u);  // never with the planned sizes: more values than slots
-    return false;
-}
 
 template <typename K>
 __global__ void __launch_bounds__(512) k_dict_collect(DictArgs a) {
@@ -152,45 +100,7 @@ __global__ void __launch_bounds__(512) k_dict_collect(DictArgs a) {
         return;
     }
     if (ld_volatile(a.overflow)) return;
-    for (uint32_t s = threadIdx.x; s < kDictCtaSlots; s += blockDim.x) {
-        if (sst[s] != 2 || ld_volatile(a.overflow)) continue;
-        DictSlot* t = a.table;
-        uint32_t g = dict_hash(skey[s]) & (kDictSlots - 1);
-        bool done = false;
-        for (uint32_t probe = 0; probe < kDictSlots && !done; ++probe) {
-            uint32_t state = ld_volatile(&t[g].state);
-            if (state == 0) {
-                state = atomicCAS(&t[g].state, 0u, 1u);
-                if (state == 0) {
-                    t[g].key = skey[s];
-                    atomicAdd(&t[g].count, scnt[s]);
-                    __threadfence();
-                    atomicExch(&t[g].state, 2u);
-                    if (atomicAdd(a.distinct, 1u) >= kDictMax) atomicOr(a.overflow, 1u);
-                    done = true;
-                    break;
-                }
-            }
-            uint32_t spins = 0;
-            while (state != 2) {
-                if (++spins > limit) {
-                    atomicOr(a.err, ERR_LOOKBACK_TIMEOUT);
-                    atomicOr(a.overflow, 1u);
-                    return;
-                }
-                if (spins > 16) __nanosleep(32);
-                state = ld_volatile(&t[g].state);
-            }
-            __threadfence();
-            if (ld_volatile(&t[g].key) == skey[s]) {
-                atomicAdd(&t[g].count, scnt[s]);
-                done = true;
-                break;
-            }
-            g = (g + 1) & (kDictSlots - 1);
-        }
-        if (!done) atomicOr(a.overflow, 1u);
-    }
+    dict_merge(skey, scnt, sst, a, limit);
 }
 
 // One CTA of 1024 threads: ranks, bin starts, lookup table, plan word.
@@ -223,8 +133,9 @@ __global__ void __launch_bounds__(1024) k_dict_rank(DictArgs a) {
     }
     __syncthreads();
     const uint32_t d = m;
-    // every row counted exactly once, or the plan does not apply
-    if (d == 0 || d > kDictMax || total != a.n) {
+    // every row counted exactly once (unless only the values were collected),
+    // or the plan does not apply
+    if (d == 0 || d > kDictMax || (a.counted && total != a.n)) {
         if (tid == 0) *a.state = a.fail_state;
         return;
     }
@@ -233,6 +144,7 @@ __global__ void __launch_bounds__(1024) k_dict_rank(DictArgs a) {
         const unsigned long long x = dk[tid];
         for (uint32_t j = 0; j < d; ++j) rank += dk[j] < x ? 1u : 0u;
         bycnt[rank] = dc[tid];
+        if (a.sorted) a.sorted[rank] = x;
     }
     for (uint32_t s = tid; s < kDictLutSlots; s += blockDim.x) a.lut->rank[s] = kDictEmpty;
     __syncthreads();
@@ -254,7 +166,7 @@ __global__ void __launch_bounds__(1024) k_dict_rank(DictArgs a) {
     if (tid < kDictMax) {
         uint32_t base = 0;
         for (int w = 0; w < (int)(tid >> 5); ++w) base += wsum[w];
-        a.bin_offsets[tid] = base + bycnt[tid];
+        if (a.bin_offsets) a.bin_offsets[tid] = base + bycnt[tid];
     }
     // lookup table: claim a free rank slot, then write the key
     if (tid < d) {
@@ -270,6 +182,7 @@ __global__ void __launch_bounds__(1024) k_dict_rank(DictArgs a) {
     }
     if (tid == 0) {
         *a.state = 2;
+        if (a.ndist) *a.ndist = d;
         if (a.taken) atomicAdd(a.taken, 1u);
     }
 }

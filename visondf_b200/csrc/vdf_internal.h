@@ -111,6 +111,11 @@ struct DictArgs {
     uint32_t* taken;          // non-null: incremented when the dictionary pass is taken
     uint32_t spin_limit;
     uint32_t* err;
+    // values without row counts (vdf_dictagg.cu): no check of the counts, and
+    // the order images in rank order with their number
+    int counted = 1;
+    unsigned long long* sorted = nullptr;
+    uint32_t* ndist = nullptr;
 };
 cudaError_t dict_collect(const DictArgs& a, cudaStream_t s);
 cudaError_t dict_rank(const DictArgs& a, cudaStream_t s);
@@ -395,6 +400,30 @@ cudaError_t prepare_segreduce_kernels();
 // The workspace holds the tile aggregates (segreduce_workspace_bytes).
 cudaError_t run_segreduce(SegArgs a, unsigned char* ws, cudaStream_t s, Profiler* prof = nullptr,
                           int* launches = nullptr);
+
+// ---- group-by without a sort, for few distinct keys (vdf_dictagg.cu) --------
+// Columns, outputs and the error word in `seg` (one key, rows in any order);
+// order 0 ascending groups, 1 and 2 descending.
+struct DictAggPlan {
+    SegArgs seg;
+    int order;
+    uint32_t spin_limit;
+    uint32_t* taken;   // device word, incremented when the groups were written
+};
+// What the launches left in the workspace's first words.
+struct DictAggWords {
+    uint32_t state;    // 2: the groups are written, unless missed is set
+    uint32_t missed;   // rows whose key was not among the collected values
+    uint32_t ndist;    // distinct keys
+    uint32_t overflow; // more than kDictMax values (or a wait gave up)
+};
+size_t dict_agg_workspace_bytes();
+cudaError_t prepare_dict_agg_kernels();
+// Collects the key's values from every row (sample false) or from one row in
+// 32, ranks them and aggregates all rows in one pass.  Asynchronous; the
+// DictAggWords sit at the workspace's start.
+cudaError_t run_dict_agg(const DictAggPlan& p, bool sample, unsigned char* ws, cudaStream_t s,
+                         Profiler* prof = nullptr, int* launches = nullptr);
 
 // ---- transform output (aggregate broadcast to rows) --------------------------
 cudaError_t run_broadcast(const uint32_t* row_group, uint64_t n, const void* group_vals, uint64_t n_groups,

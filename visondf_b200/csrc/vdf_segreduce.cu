@@ -51,11 +51,6 @@ __device__ __forceinline__ uint64_t load_raw(const void* src, int w, uint64_t i)
     return w == 4 ? (uint64_t)__ldg(static_cast<const uint32_t*>(src) + i)
                   : (uint64_t)__ldg(static_cast<const unsigned long long*>(src) + i);
 }
-__device__ __forceinline__ void store_raw(void* dst, int w, uint64_t i, uint64_t v) {
-    if (w == 4) static_cast<uint32_t*>(dst)[i] = (uint32_t)v;
-    else static_cast<unsigned long long*>(dst)[i] = v;
-}
-
 // Rows row0 .. row0+ITEMS-1 of a column into arr[j][c] (raw bits, zero-
 // extended), with 16-byte vector loads when the rows are in bounds and
 // aligned (row0 is a multiple of ITEMS; tile starts are multiples of it).
@@ -188,36 +183,6 @@ __device__ __forceinline__ Agg<NV> agg_shfl(const Agg<NV>& a, int src) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) r.w[v][q] = __shfl_sync(0xffffffffu, a.w[v][q], src);
     return r;
-}
-
-template <int NV>
-__device__ __forceinline__ void emit_group(const SegArgs& a, uint32_t g, uint32_t cnt, const uint64_t (*w)[4],
-                                           const int* vc) {
-    if (a.count_out) a.count_out[g] = (int64_t)cnt;
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-        const SegAggOut& o = a.agg[v];
-        const int dt = a.val[v].dtype;
-        if (vc[v] == VC_FLOAT) {
-            const double s = __dadd_rn(as_f(w[v][0]), as_f(w[v][1]));
-            if (o.sum) static_cast<double*>(o.sum)[g] = s;
-            if (o.mean) o.mean[g] = s / (double)cnt;
-            if (dt == F64) {
-                if (o.min) static_cast<double*>(o.min)[g] = as_f(w[v][2]);
-                if (o.max) static_cast<double*>(o.max)[g] = as_f(w[v][3]);
-            } else {
-                if (o.min) static_cast<float*>(o.min)[g] = (float)as_f(w[v][2]);
-                if (o.max) static_cast<float*>(o.max)[g] = (float)as_f(w[v][3]);
-            }
-        } else {
-            if (o.sum) static_cast<int64_t*>(o.sum)[g] = (int64_t)w[v][0];
-            if (o.sum_hi) o.sum_hi[g] = (int64_t)w[v][1];
-            if (o.mean) o.mean[g] = i128_to_double(w[v][0], w[v][1], vc[v] == VC_SINT) / (double)cnt;
-            const int wd = dtype_width(dt);
-            if (o.min) store_raw(o.min, wd, g, w[v][2]);
-            if (o.max) store_raw(o.max, wd, g, w[v][3]);
-        }
-    }
 }
 
 // Rows per lane of a warp tile: more rows amortise the tile's look-back;
