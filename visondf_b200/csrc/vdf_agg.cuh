@@ -74,35 +74,37 @@ __device__ __forceinline__ void store_raw(void* dst, int w, uint64_t i, uint64_t
     else static_cast<unsigned long long*>(dst)[i] = v;
 }
 
+// Group g's aggregates of one value column (dtype dt, accumulator words w).
+__device__ __forceinline__ void emit_column(const SegAggOut& o, int dt, uint32_t g, uint32_t cnt, const uint64_t* w,
+                                            int vc) {
+    if (vc == VC_FLOAT) {
+        const double s = __dadd_rn(as_f(w[0]), as_f(w[1]));
+        if (o.sum) static_cast<double*>(o.sum)[g] = s;
+        if (o.mean) o.mean[g] = s / (double)cnt;
+        if (dt == F64) {
+            if (o.min) static_cast<double*>(o.min)[g] = as_f(w[2]);
+            if (o.max) static_cast<double*>(o.max)[g] = as_f(w[3]);
+        } else {
+            if (o.min) static_cast<float*>(o.min)[g] = (float)as_f(w[2]);
+            if (o.max) static_cast<float*>(o.max)[g] = (float)as_f(w[3]);
+        }
+    } else {
+        if (o.sum) static_cast<int64_t*>(o.sum)[g] = (int64_t)w[0];
+        if (o.sum_hi) o.sum_hi[g] = (int64_t)w[1];
+        if (o.mean) o.mean[g] = i128_to_double(w[0], w[1], vc == VC_SINT) / (double)cnt;
+        const int wd = dtype_width(dt);
+        if (o.min) store_raw(o.min, wd, g, w[2]);
+        if (o.max) store_raw(o.max, wd, g, w[3]);
+    }
+}
+
 // Group g's record into the output columns.
 template <int NV>
 __device__ __forceinline__ void emit_group(const SegArgs& a, uint32_t g, uint32_t cnt, const uint64_t (*w)[4],
                                            const int* vc) {
     if (a.count_out) a.count_out[g] = (int64_t)cnt;
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
-        const SegAggOut& o = a.agg[v];
-        const int dt = a.val[v].dtype;
-        if (vc[v] == VC_FLOAT) {
-            const double s = __dadd_rn(as_f(w[v][0]), as_f(w[v][1]));
-            if (o.sum) static_cast<double*>(o.sum)[g] = s;
-            if (o.mean) o.mean[g] = s / (double)cnt;
-            if (dt == F64) {
-                if (o.min) static_cast<double*>(o.min)[g] = as_f(w[v][2]);
-                if (o.max) static_cast<double*>(o.max)[g] = as_f(w[v][3]);
-            } else {
-                if (o.min) static_cast<float*>(o.min)[g] = (float)as_f(w[v][2]);
-                if (o.max) static_cast<float*>(o.max)[g] = (float)as_f(w[v][3]);
-            }
-        } else {
-            if (o.sum) static_cast<int64_t*>(o.sum)[g] = (int64_t)w[v][0];
-            if (o.sum_hi) o.sum_hi[g] = (int64_t)w[v][1];
-            if (o.mean) o.mean[g] = i128_to_double(w[v][0], w[v][1], vc[v] == VC_SINT) / (double)cnt;
-            const int wd = dtype_width(dt);
-            if (o.min) store_raw(o.min, wd, g, w[v][2]);
-            if (o.max) store_raw(o.max, wd, g, w[v][3]);
-        }
-    }
+    for (int v = 0; v < NV; ++v) emit_column(a.agg[v], a.val[v].dtype, g, cnt, w[v], vc[v]);
 }
 
 }  // namespace vdf

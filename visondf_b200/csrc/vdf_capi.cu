@@ -107,6 +107,10 @@ vdf_status primary_first(vdf_ctx* c, uint64_t n, const int32_t* dts, const void*
     return VDF_OK;
 }
 
+bool small_frame(const vdf_ctx* c, const vdf::SortPlan& p);
+vdf::SmallArgs small_sort_args(vdf_ctx* c, uint64_t n, const vdf_col* keys, int nkeys, int order,
+                               const uint32_t* perm_in, uint32_t* perm_out, void* const* sorted_keys_out);
+
 vdf_status sort_impl(vdf_ctx* c, uint64_t n, const vdf_col* keys, int nkeys, int order, uint32_t* perm_out,
                      void* const* sorted_keys_out, unsigned char* ws, size_t ws_bytes, cudaStream_t s) {
     int32_t dts[vdf::kMaxKeys];
@@ -118,6 +122,12 @@ vdf_status sort_impl(vdf_ctx* c, uint64_t n, const vdf_col* keys, int nkeys, int
     vdf::SortPlan p = vdf::make_sort_plan(n, dts, nkeys, c->tuning);
     if (ws_bytes < p.ws_bytes)
         return fail(c, VDF_ERR_WORKSPACE, "workspace of %zu bytes < %zu needed", ws_bytes, p.ws_bytes);
+    if (small_frame(c, p)) {
+        const cudaError_t e =
+            vdf::run_small(small_sort_args(c, n, keys, nkeys, order, nullptr, perm_out, sorted_keys_out), s, prof_of(c));
+        c->launches++;
+        return from_cuda(c, e, "small sort");
+    }
     void* key0_out = sorted_keys_out ? sorted_keys_out[0] : nullptr;
     bool done = false;
     vdf_status pst = primary_first(c, n, dts, cols, nkeys, order, perm_out, key0_out, ws, ws_bytes, s, nullptr, &done);
@@ -131,11 +141,15 @@ vdf_status sort_impl(vdf_ctx* c, uint64_t n, const vdf_col* keys, int nkeys, int
 
 vdf_status finish_groups(vdf_ctx* c, uint64_t* n_groups_dev, uint64_t* n_groups_host, cudaStream_t s) {
     if (!n_groups_host) return VDF_OK;
-    const uint64_t* src = n_groups_dev ? n_groups_dev : count_word(c);
-    cudaError_t e = cudaMemcpyAsync(&c->host_pinned[0], src, sizeof(uint64_t), cudaMemcpyDeviceToHost, s);
+    vdf_status st;
+    if (!n_groups_dev || n_groups_dev == count_word(c)) {  // the count sits beside the error bits: one copy
+        if ((st = drain_and_check(c, s, 16)) != VDF_OK) return st;
+        std::memcpy(n_groups_host, mirror(c) + 8, sizeof(uint64_t));
+        return VDF_OK;
+    }
+    cudaError_t e = cudaMemcpyAsync(&c->host_pinned[0], n_groups_dev, sizeof(uint64_t), cudaMemcpyDeviceToHost, s);
     if (e != cudaSuccess) return from_cuda(c, e, "read group count");
-    vdf_status st = drain_and_check(c, s);
-    if (st != VDF_OK) return st;
+    if ((st = drain_and_check(c, s)) != VDF_OK) return st;
     *n_groups_host = c->host_pinned[0];
     return VDF_OK;
 }
@@ -373,6 +387,7 @@ vdf_status vdf_ctx_create(int device, vdf_ctx** out) {
             if (e == cudaSuccess) e = vdf::prepare_segreduce_kernels();
             if (e == cudaSuccess) e = vdf::prepare_batch_kernels();
             if (e == cudaSuccess) e = vdf::prepare_dict_agg_kernels();
+            if (e == cudaSuccess) e = vdf::prepare_small_kernels();
             if (e != cudaSuccess) {
                 delete c;
                 return VDF_ERR_DEVICE;
@@ -380,8 +395,9 @@ vdf_status vdf_ctx_create(int device, vdf_ctx** out) {
             g_prepared[device] = true;
         }
     }
-    if (cudaMalloc(&c->dev_small, 256) != cudaSuccess || cudaMemset(c->dev_small, 0, 256) != cudaSuccess ||
-        cudaMallocHost(&c->host_pinned, 8 * sizeof(uint64_t)) != cudaSuccess) {
+    const size_t small_bytes = kSmallGroups + vdf::dict_agg_zeroed_bytes();
+    if (cudaMalloc(&c->dev_small, small_bytes) != cudaSuccess || cudaMemset(c->dev_small, 0, small_bytes) != cudaSuccess ||
+        cudaMallocHost(&c->host_pinned, kPinnedBytes) != cudaSuccess) {
         cudaGetLastError();
         if (c->dev_small) cudaFree(c->dev_small);
         delete c;
@@ -568,6 +584,64 @@ vdf_status vdf_groupby_sorted(vdf_ctx* c, uint64_t n, const vdf_col* keys, int n
 
 namespace {
 
+// Whether a sort goes to the one-launch kernel for small frames
+// (vdf_small.cu): up to kSmallRows rows planned as LSD passes with the default
+// pass variants (a variant someone chose runs; so do the tests' stalls).
+bool small_frame(const vdf_ctx* c, const vdf::SortPlan& p) {
+    const vdf::SortTuning d = vdf::default_sort_tuning();
+    return p.n <= vdf::kSmallRows && !p.msd && !p.dict && c->tuning.variant32 == d.variant32 &&
+           c->tuning.variant64 == d.variant64 && c->tuning.stall_tile == d.stall_tile;
+}
+
+// The sort part of vdf::SmallArgs.
+vdf::SmallArgs small_sort_args(vdf_ctx* c, uint64_t n, const vdf_col* keys, int nkeys, int order,
+                               const uint32_t* perm_in, uint32_t* perm_out, void* const* sorted_keys_out) {
+    vdf::SmallArgs a{};
+    a.n = (uint32_t)n;
+    a.order = order;
+    a.perm_in = perm_in;
+    a.perm_out = perm_out;
+    a.seg.n = n;
+    a.seg.nkeys = nkeys;
+    a.seg.err = err_word(c);
+    for (int k = 0; k < nkeys; ++k) {
+        a.seg.key[k] = vdf::SegCol{keys[k].data, keys[k].dtype};
+        a.skey_out[k] = sorted_keys_out ? sorted_keys_out[k] : nullptr;
+    }
+    return a;
+}
+
+// vdf_sort_groupby of a small frame, arguments checked.
+vdf_status sort_groupby_small(vdf_ctx* c, const vdf_sort_groupby_args* x, cudaStream_t s) {
+    vdf::SmallArgs a =
+        small_sort_args(c, x->n, x->keys, x->nkeys, x->order, x->perm_in, x->perm_out, x->sorted_keys_out);
+    a.npay = x->npayload;
+    for (int p = 0; p < x->npayload; ++p) {
+        a.pay_src[p] = x->payload[p].data;
+        a.pay_dst[p] = x->payload_out ? x->payload_out[p] : nullptr;
+        a.pay_dtype[p] = x->payload[p].dtype;
+    }
+    a.groupby = x->groupby ? 1 : 0;
+    if (x->groupby) {
+        a.seg.nvals = x->nagg;
+        for (int k = 0; k < x->nkeys; ++k) a.seg.key_out[k] = x->group_keys_out ? x->group_keys_out[k] : nullptr;
+        for (int i = 0; i < x->nagg; ++i) {
+            a.val_pay[i] = x->agg_cols[i];
+            a.seg.val[i].dtype = x->payload[x->agg_cols[i]].dtype;
+            const vdf_agg_out& o = x->aggs[i];
+            a.seg.agg[i] = vdf::SegAggOut{o.sum, o.sum_hi, o.min, o.max, o.mean};
+        }
+        a.seg.count_out = x->group_count_out;
+        a.seg.group_start = x->group_start_out;
+        a.seg.row_group = x->row_group_out;
+        a.seg.n_groups = x->n_groups_dev ? x->n_groups_dev : (x->n_groups_host ? count_word(c) : nullptr);
+    }
+    const cudaError_t e = vdf::run_small(a, s, prof_of(c));
+    c->launches++;
+    if (e != cudaSuccess) return from_cuda(c, e, "small frame");
+    return x->groupby ? finish_groups(c, a.seg.n_groups, x->n_groups_host, s) : VDF_OK;
+}
+
 // Whether a call asks only for the group table of one key and synchronises
 // for the group count anyway, so that a group-by without a sort can be tried
 // (vdf_dictagg.cu), from the row count the dictionary plan of a sort is tried
@@ -618,15 +692,12 @@ vdf_status groups_without_sort(vdf_ctx* c, const vdf_sort_groupby_args* x, cudaS
     c->dict_sorts++;
     for (int sample = 1; sample >= 0; --sample) {
         int launched = 0;
-        cudaError_t e = vdf::run_dict_agg(p, sample != 0, c->ws, s, prof_of(c), &launched);
+        cudaError_t e = vdf::run_dict_agg(p, sample != 0, c->dev_small + kSmallGroups, c->ws, s, prof_of(c), &launched);
         c->launches += launched;
         if (e != cudaSuccess) return from_cuda(c, e, "group-by of few keys");
-        static_assert(sizeof(vdf::DictAggWords) == 16, "two spare host words");
-        e = cudaMemcpyAsync(&c->host_pinned[6], c->ws, sizeof(vdf::DictAggWords), cudaMemcpyDeviceToHost, s);
-        if (e != cudaSuccess) return from_cuda(c, e, "read group words");
-        if ((st = drain_and_check(c, s)) != VDF_OK) return st;
+        if ((st = drain_and_check(c, s, kMirrorBytes)) != VDF_OK) return st;
         vdf::DictAggWords w;
-        std::memcpy(&w, &c->host_pinned[6], sizeof w);
+        std::memcpy(&w, mirror(c) + kSmallGroups, sizeof w);
         if (w.state == 2 && !w.missed) {
             *x->n_groups_host = w.ndist;
             *done = true;
@@ -679,6 +750,7 @@ vdf_status sort_groupby_locked(vdf_ctx* c, const vdf_sort_groupby_args* x, cudaS
         tuning.dict = 0;  // the key takes too many values for the dictionary plan
     }
     const vdf::SortPlan plan = vdf::make_sort_plan(n, dts, x->nkeys, tuning);
+    if (small_frame(c, plan)) return sort_groupby_small(c, x, s);
     // Sorted copies needed by the group-by that the caller did not ask for
     // live in the workspace: [perm][key 0][keys 1..][aggregated payload][tail]
     // where tail = max(sort workspace, group-by workspace).
@@ -1098,16 +1170,6 @@ vdf_status vdf_broadcast(vdf_ctx* c, uint64_t n, const uint32_t* row_group, cons
                      "broadcast");
 }
 
-// Reads a device count (u64) into *host after the stream's work.
-static vdf_status read_count(vdf_ctx* c, const uint64_t* dev, uint64_t* host, cudaStream_t s, const char* what) {
-    if (!host) return VDF_OK;
-    cudaError_t e = cudaMemcpyAsync(&c->host_pinned[0], dev, sizeof(uint64_t), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return from_cuda(c, e, what);
-    *host = c->host_pinned[0];
-    return drain_and_check(c, s);
-}
-
 // vdf_unique with the context lock held
 static vdf_status unique_locked(vdf_ctx* c, uint64_t n, vdf_col key, int keep_last, uint8_t* keep_out,
                                 uint64_t* n_unique_dev, uint64_t* n_unique_host, void* stream) {
@@ -1124,14 +1186,14 @@ static vdf_status unique_locked(vdf_ctx* c, uint64_t n, vdf_col key, int keep_la
     }
     if (!keep_out) return fail(c, VDF_ERR_INVALID_ARG, "keep_out is NULL");
     const int w = vdf::dtype_width(key.dtype);
-    // workspace: permutation | sorted keys | count | mark bits | the sort's own
-    const size_t o_perm = 0, o_keys = align256(4 * n), o_cnt = o_keys + align256((size_t)w * n);
-    const size_t o_bits = o_cnt + 256, o_sort = o_bits + align256(vdf::unique_workspace_bytes(n));
+    // workspace: permutation | sorted keys | mark bits | the sort's own
+    const size_t o_perm = 0, o_keys = align256(4 * n), o_bits = o_keys + align256((size_t)w * n);
+    const size_t o_sort = o_bits + align256(vdf::unique_workspace_bytes(n));
     const vdf::SortPlan plan = vdf::make_sort_plan(n, &key.dtype, 1, c->tuning);
     if ((st = ws_ensure(c, o_sort + sort_ws_need(plan, n, 1, nullptr))) != VDF_OK) return st;
     uint32_t* perm = reinterpret_cast<uint32_t*>(c->ws + o_perm);
     void* skeys = c->ws + o_keys;
-    uint64_t* cnt = n_unique_dev ? n_unique_dev : reinterpret_cast<uint64_t*>(c->ws + o_cnt);
+    uint64_t* cnt = n_unique_dev ? n_unique_dev : count_word(c);
     void* const souts[1] = {skeys};
     if ((st = sort_impl(c, n, &key, 1, VDF_ORDER_ASC, perm, souts, c->ws + o_sort, c->ws_cap - o_sort, s)) != VDF_OK)
         return st;
@@ -1142,7 +1204,7 @@ static vdf_status unique_locked(vdf_ctx* c, uint64_t n, vdf_col key, int keep_la
                                  err_word(c), s);
     c->launches += 2;
     if (e != cudaSuccess) return from_cuda(c, e, "unique");
-    return read_count(c, cnt, n_unique_host, s, "read unique count");
+    return finish_groups(c, cnt, n_unique_host, s);
 }
 
 // vdf_left_join_index with the context lock held
@@ -1163,12 +1225,12 @@ static vdf_status left_join_locked(vdf_ctx* c, uint64_t n_left, vdf_col left_key
     const uint64_t nr = n_right, nl = n_left;
     const bool aligned = method == VDF_JOIN_ALIGNED;
     // workspace: right permutation | right sorted keys | distinct keys | run
-    // starts | group count | matched count | (aligned: left permutation, left
+    // starts | group count | (aligned: left permutation, left
     // sorted keys, run of each sorted left row, left run starts, left group
     // count) | the sorts', the reductions' or the hash table's own
     const size_t o_perm = 0, o_sk = align256(4 * nr), o_uk = o_sk + align256((size_t)w * nr);
-    const size_t o_gs = o_uk + align256((size_t)w * nr), o_ng = o_gs + align256(4 * nr), o_cnt = o_ng + 256;
-    size_t o = o_cnt + 256;
+    const size_t o_gs = o_uk + align256((size_t)w * nr), o_ng = o_gs + align256(4 * nr);
+    size_t o = o_ng + 256;
     size_t o_lperm = 0, o_lsk = 0, o_lrg = 0, o_lgs = 0, o_lng = 0;
     if (aligned) {
         o_lperm = o; o += align256(4 * nl);
@@ -1189,13 +1251,13 @@ static vdf_status left_join_locked(vdf_ctx* c, uint64_t n_left, vdf_col left_key
         tail = std::max(tail, std::max(sort_ws_need(plan, nl, 1, nullptr), vdf::segreduce_workspace_bytes(nl, 0)));
     }
     if ((st = ws_ensure(c, o_tail + tail)) != VDF_OK) return st;
-    uint64_t* cnt = n_matched_dev ? n_matched_dev : reinterpret_cast<uint64_t*>(c->ws + o_cnt);
+    uint64_t* cnt = n_matched_dev ? n_matched_dev : count_word(c);
     cudaError_t e = cudaMemsetAsync(cnt, 0, sizeof(uint64_t), s);
     if (e != cudaSuccess) return from_cuda(c, e, "clear count");
-    if (nl == 0) return read_count(c, cnt, n_matched_host, s, "read match count");
+    if (nl == 0) return finish_groups(c, cnt, n_matched_host, s);
     if (nr == 0) {  // nothing to match
         if ((e = cudaMemsetAsync(match_out, 0xff, 4 * nl, s)) != cudaSuccess) return from_cuda(c, e, "no match");
-        return read_count(c, cnt, n_matched_host, s, "read match count");
+        return finish_groups(c, cnt, n_matched_host, s);
     }
     // one side: stable sort, then its distinct keys and their run starts
     auto sort_side = [&](uint64_t n, const vdf_col& key, size_t o_p, size_t o_s, size_t o_u, size_t o_g, size_t o_n,
@@ -1239,7 +1301,7 @@ static vdf_status left_join_locked(vdf_ctx* c, uint64_t n_left, vdf_col left_key
     }
     c->launches += 2;
     if (e != cudaSuccess) return from_cuda(c, e, "join");
-    return read_count(c, cnt, n_matched_host, s, "read match count");
+    return finish_groups(c, cnt, n_matched_host, s);
 }
 
 vdf_status vdf_unique(vdf_ctx* c, uint64_t n, vdf_col key, int keep_last, uint8_t* keep_out,

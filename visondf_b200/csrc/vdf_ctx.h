@@ -6,6 +6,7 @@
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
+#include <cstring>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -79,10 +80,12 @@ struct vdf_ctx {
     size_t ws_cap = 0;
     unsigned char* dev_small = nullptr;  // [0,4): error bits; [8,16): group count scratch;
                                          // [16,20): tie flag; [24,28): MSD fallbacks;
-                                         // [28,32): dictionary passes taken
+                                         // [28,32): dictionary passes taken; from kSmallGroups:
+                                         // words and tables of the group-by without a sort
     uint64_t* host_pinned = nullptr;     // [0]: group count, [1]: error bits, [2]: tie flag, [3]: fallbacks,
                                          // [4]: pivot key counts (two words), [5]: dictionary passes
-                                         // taken, [6..7] spare
+                                         // taken, [6..7] spare, [8..]: copy of dev_small's first
+                                         // kMirrorBytes bytes (error bits, counts, group words)
     uint64_t msd_sorts = 0;              // sorts planned MSD-first
     uint64_t dict_sorts = 0;             // sorts that tried the dictionary plan
     uint32_t emit_min_heads = 0;         // group-by emit: striped-path threshold (0 = default)
@@ -131,6 +134,9 @@ inline size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 
 inline vdf::Profiler* prof_of(vdf_ctx* c) { return c->profiling ? &c->prof : nullptr; }
 
+constexpr size_t kSmallGroups = 64;  // offset in dev_small of the group-by words (vdf::DictAggWords)
+constexpr size_t kMirrorBytes = kSmallGroups + sizeof(vdf::DictAggWords);
+constexpr size_t kPinnedBytes = 8 * sizeof(uint64_t) + (kMirrorBytes + 63) / 64 * 64;
 inline uint32_t* err_word(vdf_ctx* c) { return reinterpret_cast<uint32_t*>(c->dev_small); }
 inline uint64_t* count_word(vdf_ctx* c) { return reinterpret_cast<uint64_t*>(c->dev_small + 8); }
 inline uint32_t* tie_word(vdf_ctx* c) { return reinterpret_cast<uint32_t*>(c->dev_small + 16); }
@@ -191,12 +197,16 @@ inline vdf_status io_ensure(vdf_ctx* c, size_t bytes) {
 // vdf_sort_groupby on device pointers with the context lock already held.
 vdf_status sort_groupby_device(vdf_ctx* c, const vdf_sort_groupby_args* x, cudaStream_t s);
 
-// Reads and clears the device error bits after the stream has drained.
-inline vdf_status drain_and_check(vdf_ctx* c, cudaStream_t s) {
-    cudaError_t e = cudaMemcpyAsync(&c->host_pinned[1], err_word(c), sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+// Reads and clears the device error bits after the stream has drained; the
+// first `bytes` bytes of the small device words come along in one copy
+// (mirror(c)).
+inline const unsigned char* mirror(const vdf_ctx* c) { return reinterpret_cast<const unsigned char*>(c->host_pinned + 8); }
+inline vdf_status drain_and_check(vdf_ctx* c, cudaStream_t s, size_t bytes = sizeof(uint32_t)) {
+    cudaError_t e = cudaMemcpyAsync(c->host_pinned + 8, c->dev_small, bytes, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return from_cuda(c, e, "stream synchronize");
-    uint32_t bits = (uint32_t)c->host_pinned[1];
+    uint32_t bits;
+    std::memcpy(&bits, mirror(c), sizeof bits);
     if (bits) {
         cudaMemsetAsync(err_word(c), 0, sizeof(uint32_t), s);
         cudaStreamSynchronize(s);

@@ -542,17 +542,16 @@ int sm_count() {
     return sms;
 }
 
-// workspace: words | collection table | lookup table | sorted values | partials
+// cleared words: DictAggWords | number of values | collection table
+constexpr size_t kZeroTable = (sizeof(DictAggWords) + 4 + 15) / 16 * 16;
+constexpr size_t kZeroBytes = kZeroTable + sizeof(DictSlot) * kDictSlots;
+// workspace: lookup table | sorted values | partials
 struct AggLayout {
-    size_t words, distinct, table, zero_bytes, lut, sorted, parts, total;
+    size_t lut, sorted, parts, total;
 };
 AggLayout agg_layout(int ctas) {
     AggLayout L{};
     size_t o = 0;
-    L.words = o; o += sizeof(DictAggWords);
-    L.distinct = o; o = align_up(o + 4, 256);
-    L.table = o; o = align_up(o + sizeof(DictSlot) * kDictSlots, 256);
-    L.zero_bytes = o;
     L.lut = o; o = align_up(o + sizeof(DictLut), 256);
     L.sorted = o; o = align_up(o + 8 * kDictMax, 256);
     L.parts = o; o = align_up(o + (size_t)ctas * kDictMax * sizeof(AggPart), 256);
@@ -565,6 +564,8 @@ static_assert(kAggTables + (size_t)(kDictMax + 1) * (kMaxVals * 16 + 16 * kMaxVa
               "accumulators of one warp per column");
 }  // namespace
 
+size_t dict_agg_zeroed_bytes() { return kZeroBytes; }
+
 size_t dict_agg_workspace_bytes() { return agg_layout(sm_count()).total; }
 
 cudaError_t prepare_dict_agg_kernels() {
@@ -574,23 +575,23 @@ cudaError_t prepare_dict_agg_kernels() {
     return e;
 }
 
-cudaError_t run_dict_agg(const DictAggPlan& p, bool sample, unsigned char* ws, cudaStream_t s, Profiler* prof,
+cudaError_t run_dict_agg(const DictAggPlan& p, bool sample, unsigned char* zeroed, unsigned char* ws, cudaStream_t s, Profiler* prof,
                          int* launches) {
     const SegArgs& g = p.seg;
     const int sms = sm_count();
     const AggLayout L = agg_layout(sms);
     const int width = dtype_width(g.key[0].dtype);
-    cudaError_t e = cudaMemsetAsync(ws, 0, L.zero_bytes, s);
+    cudaError_t e = cudaMemsetAsync(zeroed, 0, kZeroBytes, s);
     if (e != cudaSuccess) return e;
-    DictAggWords* words = reinterpret_cast<DictAggWords*>(ws + L.words);
+    DictAggWords* words = reinterpret_cast<DictAggWords*>(zeroed);
     DictArgs da{};
     da.keys = g.key[0].src;
     da.dtype = g.key[0].dtype;
     da.invert = p.order == 1 ? 1 : 0;
     da.width = width;
     da.n = g.n;
-    da.table = reinterpret_cast<DictSlot*>(ws + L.table);
-    da.distinct = reinterpret_cast<uint32_t*>(ws + L.distinct);
+    da.table = reinterpret_cast<DictSlot*>(zeroed + kZeroTable);
+    da.distinct = reinterpret_cast<uint32_t*>(zeroed + sizeof(DictAggWords));
     da.overflow = &words->overflow;
     da.state = &words->state;
     da.fail_state = 1;

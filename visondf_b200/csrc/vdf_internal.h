@@ -410,20 +410,45 @@ struct DictAggPlan {
     uint32_t spin_limit;
     uint32_t* taken;   // device word, incremented when the groups were written
 };
-// What the launches left in the workspace's first words.
+// What the launches left in the first cleared words.
 struct DictAggWords {
     uint32_t state;    // 2: the groups are written, unless missed is set
     uint32_t missed;   // rows whose key was not among the collected values
     uint32_t ndist;    // distinct keys
     uint32_t overflow; // more than kDictMax values (or a wait gave up)
 };
+size_t dict_agg_zeroed_bytes();     // words and collection table, cleared by every run
 size_t dict_agg_workspace_bytes();
 cudaError_t prepare_dict_agg_kernels();
 // Collects the key's values from every row (sample false) or from one row in
 // 32, ranks them and aggregates all rows in one pass.  Asynchronous; the
-// DictAggWords sit at the workspace's start.
-cudaError_t run_dict_agg(const DictAggPlan& p, bool sample, unsigned char* ws, cudaStream_t s,
+// DictAggWords sit at the start of `zeroed`.
+cudaError_t run_dict_agg(const DictAggPlan& p, bool sample, unsigned char* zeroed, unsigned char* ws, cudaStream_t s,
                          Profiler* prof = nullptr, int* launches = nullptr);
+
+// ---- small frames: sort, gather and group-by in one launch (vdf_small.cu) ----
+// Rows one CTA takes: what its shared memory holds with four value columns
+// (216 KB).  At that size one CTA still takes less than half the general
+// path's launches (4,000 distinct int64 keys, f64 + int64 values: 62 against
+// 136 us).
+constexpr uint32_t kSmallRows = 4096;
+struct SmallArgs {
+    // key columns, value dtypes and group outputs; val[].src is not used
+    // (values come from the payload column val_pay[v])
+    SegArgs seg;
+    uint32_t n;
+    int order, groupby;
+    const uint32_t* perm_in;
+    uint32_t* perm_out;
+    void* skey_out[kMaxKeys];
+    int npay;
+    const void* pay_src[kMaxGather];
+    void* pay_dst[kMaxGather];   // sorted copy, or null
+    int pay_dtype[kMaxGather];
+    int val_pay[kMaxVals];
+};
+cudaError_t prepare_small_kernels();
+cudaError_t run_small(const SmallArgs& a, cudaStream_t s, Profiler* prof = nullptr);
 
 // ---- transform output (aggregate broadcast to rows) --------------------------
 cudaError_t run_broadcast(const uint32_t* row_group, uint64_t n, const void* group_vals, uint64_t n_groups,
