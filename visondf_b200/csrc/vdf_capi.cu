@@ -1223,34 +1223,6 @@ static vdf_status left_join_locked(vdf_ctx* c, uint64_t n_left, vdf_col left_key
     DeviceGuard g(c->device);
     const int w = vdf::dtype_width(right_key.dtype);
     const uint64_t nr = n_right, nl = n_left;
-    const bool aligned = method == VDF_JOIN_ALIGNED;
-    // workspace: right permutation | right sorted keys | distinct keys | run
-    // starts | group count | (aligned: left permutation, left
-    // sorted keys, run of each sorted left row, left run starts, left group
-    // count) | the sorts', the reductions' or the hash table's own
-    const size_t o_perm = 0, o_sk = align256(4 * nr), o_uk = o_sk + align256((size_t)w * nr);
-    const size_t o_gs = o_uk + align256((size_t)w * nr), o_ng = o_gs + align256(4 * nr);
-    size_t o = o_ng + 256;
-    size_t o_lperm = 0, o_lsk = 0, o_lrg = 0, o_lgs = 0, o_lng = 0;
-    if (aligned) {
-        o_lperm = o; o += align256(4 * nl);
-        o_lsk = o; o += align256((size_t)w * nl);
-        o_lrg = o; o += align256(4 * nl);
-        o_lgs = o; o += align256(4 * nl);
-        o_lng = o; o += 256;
-    }
-    const size_t o_tail = o;
-    size_t tail = 0;
-    if (nr) {
-        const vdf::SortPlan plan = vdf::make_sort_plan(nr, &right_key.dtype, 1, c->tuning);
-        tail = std::max(sort_ws_need(plan, nr, 1, nullptr), vdf::segreduce_workspace_bytes(nr, 0));
-        tail = std::max(tail, vdf::join_workspace_bytes(nr));
-    }
-    if (aligned && nl) {
-        const vdf::SortPlan plan = vdf::make_sort_plan(nl, &left_key.dtype, 1, c->tuning);
-        tail = std::max(tail, std::max(sort_ws_need(plan, nl, 1, nullptr), vdf::segreduce_workspace_bytes(nl, 0)));
-    }
-    if ((st = ws_ensure(c, o_tail + tail)) != VDF_OK) return st;
     uint64_t* cnt = n_matched_dev ? n_matched_dev : count_word(c);
     cudaError_t e = cudaMemsetAsync(cnt, 0, sizeof(uint64_t), s);
     if (e != cudaSuccess) return from_cuda(c, e, "clear count");
@@ -1259,6 +1231,29 @@ static vdf_status left_join_locked(vdf_ctx* c, uint64_t n_left, vdf_col left_key
         if ((e = cudaMemsetAsync(match_out, 0xff, 4 * nl, s)) != cudaSuccess) return from_cuda(c, e, "no match");
         return finish_groups(c, cnt, n_matched_host, s);
     }
+    if (method != VDF_JOIN_ALIGNED) {  // no order needed: the right rows straight into a hash table
+        if ((st = ws_ensure(c, vdf::join_rows_workspace_bytes(nr))) != VDF_OK) return st;
+        e = vdf::run_join_rows(left_key.data, nl, right_key.data, nr, w, method == VDF_JOIN_LAST, c->ws, match_out,
+                               reinterpret_cast<unsigned long long*>(cnt), err_word(c), s);
+        c->launches += 2;
+        if (e != cudaSuccess) return from_cuda(c, e, "join");
+        return finish_groups(c, cnt, n_matched_host, s);
+    }
+    // workspace: right permutation | right sorted keys | distinct keys | run
+    // starts | group count | left permutation | left sorted keys | run of each
+    // sorted left row | left run starts | left group count | the sorts', the
+    // reductions' or the hash table's own
+    const size_t o_perm = 0, o_sk = align256(4 * nr), o_uk = o_sk + align256((size_t)w * nr);
+    const size_t o_gs = o_uk + align256((size_t)w * nr), o_ng = o_gs + align256(4 * nr);
+    const size_t o_lperm = o_ng + 256, o_lsk = o_lperm + align256(4 * nl), o_lrg = o_lsk + align256((size_t)w * nl);
+    const size_t o_lgs = o_lrg + align256(4 * nl), o_lng = o_lgs + align256(4 * nl), o_tail = o_lng + 256;
+    auto side_tail = [&](uint64_t n, const vdf_col& key) {
+        const vdf::SortPlan plan = vdf::make_sort_plan(n, &key.dtype, 1, c->tuning);
+        return std::max(sort_ws_need(plan, n, 1, nullptr), vdf::segreduce_workspace_bytes(n, 0));
+    };
+    const size_t tail =
+        std::max(std::max(side_tail(nr, right_key), side_tail(nl, left_key)), vdf::join_workspace_bytes(nr));
+    if ((st = ws_ensure(c, o_tail + tail)) != VDF_OK) return st;
     // one side: stable sort, then its distinct keys and their run starts
     auto sort_side = [&](uint64_t n, const vdf_col& key, size_t o_p, size_t o_s, size_t o_u, size_t o_g, size_t o_n,
                          size_t o_rg) -> vdf_status {
@@ -1283,22 +1278,16 @@ static vdf_status left_join_locked(vdf_ctx* c, uint64_t n_left, vdf_col left_key
         return ee == cudaSuccess ? VDF_OK : from_cuda(c, ee, "distinct keys");
     };
     if ((st = sort_side(nr, right_key, o_perm, o_sk, o_uk, o_gs, o_ng, 0)) != VDF_OK) return st;
-    if (aligned && (st = sort_side(nl, left_key, o_lperm, o_lsk, 0, o_lgs, o_lng, o_lrg)) != VDF_OK) return st;
-    const uint32_t* perm_r = reinterpret_cast<const uint32_t*>(c->ws + o_perm);
-    const uint32_t* gs_r = reinterpret_cast<const uint32_t*>(c->ws + o_gs);
+    if ((st = sort_side(nl, left_key, o_lperm, o_lsk, 0, o_lgs, o_lng, o_lrg)) != VDF_OK) return st;
     const uint64_t* ng_r = reinterpret_cast<const uint64_t*>(c->ws + o_ng);
-    e = vdf::run_join_build(c->ws + o_uk, w, gs_r, ng_r, perm_r, nr, method, c->ws + o_tail, err_word(c), s);
-    if (e == cudaSuccess) {
-        if (aligned)
-            e = vdf::run_join_probe_aligned(c->ws + o_lsk, w, reinterpret_cast<const uint32_t*>(c->ws + o_lperm),
-                                            reinterpret_cast<const uint32_t*>(c->ws + o_lrg),
-                                            reinterpret_cast<const uint32_t*>(c->ws + o_lgs), nl, c->ws + o_tail, gs_r,
-                                            ng_r, perm_r, nr, match_out, reinterpret_cast<unsigned long long*>(cnt),
-                                            err_word(c), s);
-        else
-            e = vdf::run_join_probe(left_key.data, nl, w, c->ws + o_tail, nr, match_out,
-                                    reinterpret_cast<unsigned long long*>(cnt), s);
-    }
+    e = vdf::run_join_build(c->ws + o_uk, w, ng_r, nr, c->ws + o_tail, err_word(c), s);
+    if (e == cudaSuccess)
+        e = vdf::run_join_probe_aligned(
+            c->ws + o_lsk, w, reinterpret_cast<const uint32_t*>(c->ws + o_lperm),
+            reinterpret_cast<const uint32_t*>(c->ws + o_lrg), reinterpret_cast<const uint32_t*>(c->ws + o_lgs), nl,
+            c->ws + o_tail, reinterpret_cast<const uint32_t*>(c->ws + o_gs), ng_r,
+            reinterpret_cast<const uint32_t*>(c->ws + o_perm), nr, match_out, reinterpret_cast<unsigned long long*>(cnt),
+            err_word(c), s);
     c->launches += 2;
     if (e != cudaSuccess) return from_cuda(c, e, "join");
     return finish_groups(c, cnt, n_matched_host, s);
