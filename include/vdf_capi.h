@@ -156,10 +156,10 @@ vdf_status vdf_sort_variant_info(int index, int32_t* key_width, int32_t* threads
  * the next tile's copy overlapping the current tile's ranking), on a
  * persistent grid. */
 uint32_t vdf_sort_variant_flags(int index);
-/* Group-by emit tuning: a 512-row tile with at least striped_min_heads group
- * starts is written by the striped path (the thread of each group's first
- * row walks and writes the group, consecutive threads writing consecutive
- * groups); others by the per-thread walk after a warp scan of aggregates.
+/* Group-by emit tuning: rows with at least striped_min_heads group starts per
+ * 512 are written by the striped path (the thread of each group's first row
+ * walks and writes the group); others with consecutive threads taking
+ * consecutive groups from the list of their first rows.
  * 0 restores the default (480); get returns the value in use. */
 vdf_status vdf_ctx_set_group_tuning(vdf_ctx* ctx, uint32_t striped_min_heads);
 uint32_t vdf_ctx_get_group_tuning(vdf_ctx* ctx);

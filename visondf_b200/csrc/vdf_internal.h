@@ -388,9 +388,9 @@ struct SegArgs {
     uint32_t* row_group;       // group index of each sorted row (may be null)
     uint64_t* n_groups;        // device word: number of groups (may be null)
     uint32_t* err;             // error word
-    // tiles of the emit pass with at least this many heads (of 512 rows)
-    // take the striped path, each group written by the thread of its first
-    // row; 0 = kStripedMinHeads
+    // rows of the emit pass with at least this many heads per 512 take the
+    // striped path, each group written by the thread of its first row; 0 =
+    // kStripedMinHeads
     uint32_t striped_min_heads = 0;
 };
 constexpr uint32_t kStripedMinHeads = 480;

@@ -18,11 +18,10 @@
 //   * k_seg_scan (one CTA) turns the tile aggregates into exclusive tile
 //     prefixes: the number of groups before each tile and the partial of the
 //     segment that runs into it;
-//   * k_seg_emit re-reads each tile, block-scans it seeded with its prefix,
-//     and writes every segment that ends inside it (keys, count, sum, min,
-//     max, mean), staged per warp in shared memory so that each output
-//     column is written by consecutive lanes at consecutive group ids; a
-//     tile without a segment head (known from the prefixes) is skipped.
+//   * k_seg_emit re-reads the rows, lists the segments that start in a CTA's
+//     tiles, and folds and writes each (keys, count, sum, min, max, mean) by
+//     one thread, eight lanes or a warp, depending on its length; rows
+//     without a segment head (known from the prefixes) are skipped.
 // Nothing spins on another CTA, so there is no look-back latency chain: the
 // price is one extra sequential read of the key and value columns (of the
 // tiles that hold a head).
@@ -173,116 +172,8 @@ __device__ __forceinline__ Agg<NV> agg_shfl_down(const Agg<NV>& a, int d) {
         for (int q = 0; q < 4; ++q) r.w[v][q] = __shfl_down_sync(0xffffffffu, a.w[v][q], d);
     return r;
 }
-template <int NV>
-__device__ __forceinline__ Agg<NV> agg_shfl(const Agg<NV>& a, int src) {
-    Agg<NV> r;
-    r.heads = __shfl_sync(0xffffffffu, a.heads, src);
-    r.cnt = __shfl_sync(0xffffffffu, a.cnt, src);
-#pragma unroll
-    for (int v = 0; v < NV; ++v)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) r.w[v][q] = __shfl_sync(0xffffffffu, a.w[v][q], src);
-    return r;
-}
-
-// Rows per lane of a warp tile: more rows amortise the tile's look-back;
-// fewer keep registers free when many value columns are aggregated.
-
-// Per-warp staging of completed groups (records) and new groups (keys),
-// column-major with one padding slot per 32 entries: a thread fills entries
-// ITEMS*t .. ITEMS*t+ITEMS-1 and the write-out reads consecutive entries
-// across lanes; the skew keeps both patterns (nearly) bank-conflict free.
-template <int NK, int NV, int ITEMS>
-struct WarpStage {
-    static constexpr int ROWS = ITEMS * 32;
-    static constexpr int SLOTS = ROWS + 1 + (ROWS + 1) / 32 + 1;
-    static __device__ __forceinline__ int at(uint32_t i) { return (int)(i + (i >> 5)); }
-    uint64_t w[NV > 0 ? NV : 1][4][SLOTS];
-    uint64_t key[NK][SLOTS];
-    uint32_t cnt[SLOTS];
-    uint32_t start[SLOTS];
-    __device__ __forceinline__ void put(uint32_t i, uint32_t c, const uint64_t (*src)[4]) {
-        const int x = at(i);
-        cnt[x] = c;
-#pragma unroll
-        for (int v = 0; v < NV; ++v)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) w[v][q][x] = src[v][q];
-    }
-};
-
 constexpr int kSegThreads = 256;
-constexpr int kSegItems = 2;
-constexpr int kSegTile = kSegThreads * kSegItems;  // rows per tile
-constexpr int kSegTilesPerCta = 1;                  // tiles each CTA of the reduce and emit passes takes
-
-extern __shared__ __align__(16) unsigned char seg_smem[];
-
-template <int NK, int NV>
-__host__ __device__ constexpr size_t stage_offset() {
-    return ((sizeof(Agg<NV>) * 2 * (kSegThreads / 32 + 1) + 15) / 16) * 16;
-}
-template <int NK, int NV>
-__host__ __device__ constexpr size_t emit_smem_bytes() {
-    return stage_offset<NK, NV>() + sizeof(WarpStage<NK, NV, kSegItems>) * (kSegThreads / 32);
-}
-
-// Head flags of this thread's rows (bit j: row row0 + j starts a group).
-template <int NK>
-__device__ __forceinline__ uint32_t row_heads(const SegArgs& a, uint64_t row0, int lane, const int* kw) {
-    constexpr int ITEMS = kSegItems;
-    const uint64_t n = a.n;
-    uint64_t key[ITEMS][NK];
-#pragma unroll
-    for (int k = 0; k < NK; ++k) load_rows<ITEMS>(a.key[k].src, kw[k], row0, n, key, k);
-    uint64_t prev[NK];
-#pragma unroll
-    for (int k = 0; k < NK; ++k) prev[k] = __shfl_up_sync(0xffffffffu, key[ITEMS - 1][k], 1);
-    if (lane == 0 && row0 > 0 && row0 < n) {
-#pragma unroll
-        for (int k = 0; k < NK; ++k) prev[k] = load_raw(a.key[k].src, kw[k], row0 - 1);
-    }
-    uint32_t hmask = 0;
-#pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-        const uint64_t r = row0 + j;
-        bool h = (r == 0);
-#pragma unroll
-        for (int k = 0; k < NK; ++k) h |= (j == 0 ? prev[k] : key[j - 1][k]) != key[j][k];
-        if (r < n && h) hmask |= 1u << j;
-    }
-    return hmask;
-}
-
-// The fold of this thread's rows into one aggregate, given their head flags.
-template <int NV>
-__device__ __forceinline__ Agg<NV> fold_rows(const SegArgs& a, uint64_t row0, const int* vc, uint32_t hmask) {
-    constexpr int ITEMS = kSegItems;
-    const uint64_t n = a.n;
-    uint64_t val[ITEMS][NV > 0 ? NV : 1];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) load_vals<ITEMS>(a.val[v].src, a.val[v].dtype, row0, n, val, v);
-    Agg<NV> t = agg_identity<NV>();
-#pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-        if (row0 + j >= n) break;
-        if (((hmask >> j) & 1u) || t.cnt == 0) {
-            if ((hmask >> j) & 1u) t.heads++;
-            t.cnt = 1;
-#pragma unroll
-            for (int v = 0; v < NV; ++v) col_init(t.w[v], val[j][v], vc[v]);
-        } else {
-            t.cnt++;
-#pragma unroll
-            for (int v = 0; v < NV; ++v) {
-                uint64_t one[4];
-                col_init(one, val[j][v], vc[v]);
-                col_merge(t.w[v], one, vc[v]);
-            }
-        }
-    }
-    return t;
-}
+constexpr int kSegTile = 512;  // rows per tile
 
 // Value-class patterns fixed at compile time (VCP): 0 = read from the column
 // dtypes at run time; 1 = two columns, float then signed integer (the
@@ -329,126 +220,8 @@ __device__ __forceinline__ void seg_setup(const SegArgs& a, int* vc, int* kw) {
 // threads whose rows lie in the trailing segment read values and fold them;
 // only warps overlapping it reduce.  With many groups (one per few rows)
 // almost no values are read here.
-template <int NV>
-struct TileSmem {
-    Agg<NV> s_warp[kSegThreads / 32];
-    uint32_t s_heads[kSegThreads / 32];
-    int s_last[kSegThreads / 32];
-};
-
-template <int NK, int NV>
-__device__ __forceinline__ void seg_tile_body(const SegArgs& a, Agg<NV>* tile_agg, uint32_t tile, TileSmem<NV>& sm) {
-    constexpr int ITEMS = kSegItems, WARPS = kSegThreads / 32;
-    Agg<NV>* s_warp = sm.s_warp;
-    uint32_t* s_heads = sm.s_heads;
-    int* s_last = sm.s_last;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint64_t n = a.n;
-    const uint64_t tile0 = (uint64_t)tile * kSegTile;
-    const uint64_t row0 = tile0 + (uint64_t)tid * ITEMS;
-    int vc[NV > 0 ? NV : 1], kw[NK];
-    seg_setup<NK, NV>(a, vc, kw);
-
-    // keys and head flags
-    uint64_t key[ITEMS][NK];
-#pragma unroll
-    for (int k = 0; k < NK; ++k) load_rows<ITEMS>(a.key[k].src, kw[k], row0, n, key, k);
-    uint64_t prev[NK];
-#pragma unroll
-    for (int k = 0; k < NK; ++k) prev[k] = __shfl_up_sync(0xffffffffu, key[ITEMS - 1][k], 1);
-    if (lane == 0 && row0 > 0 && row0 < n) {
-#pragma unroll
-        for (int k = 0; k < NK; ++k) prev[k] = load_raw(a.key[k].src, kw[k], row0 - 1);
-    }
-    uint32_t hmask = 0;
-#pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-        const uint64_t r = row0 + j;
-        bool h = (r == 0);
-#pragma unroll
-        for (int k = 0; k < NK; ++k) h |= (j == 0 ? prev[k] : key[j - 1][k]) != key[j][k];
-        if (r < n && h) hmask |= 1u << j;
-    }
-    // head count and the last head (row within the tile, -1 for none)
-    uint32_t heads = __popc(hmask);
-    int last = hmask ? tid * ITEMS + (31 - __clz(hmask)) : -1;
-#pragma unroll
-    for (int d = 16; d >= 1; d >>= 1) {
-        heads += __shfl_down_sync(0xffffffffu, heads, d);
-        last = max(last, __shfl_down_sync(0xffffffffu, last, d));
-    }
-    if (lane == 0) {
-        s_heads[warp] = heads;
-        s_last[warp] = last;
-    }
-    __syncthreads();
-    uint32_t tile_heads = 0;
-    int tile_last = -1;
-#pragma unroll
-    for (int w = 0; w < WARPS; ++w) {
-        tile_heads += s_heads[w];
-        tile_last = max(tile_last, s_last[w]);
-    }
-    const int from = tile_last >= 0 ? tile_last : 0;  // first row of the trailing segment
-
-    // fold this thread's rows of the trailing segment
-    Agg<NV> t = agg_identity<NV>();
-    if (tid * ITEMS + ITEMS - 1 >= from && row0 < n) {
-        uint64_t val[ITEMS][NV > 0 ? NV : 1];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) load_vals<ITEMS>(a.val[v].src, a.val[v].dtype, row0, n, val, v);
-#pragma unroll
-        for (int j = 0; j < ITEMS; ++j) {
-            if (row0 + j >= n || tid * ITEMS + j < from) continue;
-            if (t.cnt == 0) {
-#pragma unroll
-                for (int v = 0; v < NV; ++v) col_init(t.w[v], val[j][v], vc[v]);
-            } else {
-#pragma unroll
-                for (int v = 0; v < NV; ++v) {
-                    uint64_t one[4];
-                    col_init(one, val[j][v], vc[v]);
-                    col_merge(t.w[v], one, vc[v]);
-                }
-            }
-            t.cnt++;
-        }
-    }
-    // ordered reduction over the warps that hold trailing rows (lower lanes
-    // are earlier rows; heads stay 0, so the combine merges)
-    const bool active = (warp + 1) * 32 * ITEMS - 1 >= from;
-    if (active) {
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const Agg<NV> o = agg_shfl_down(t, d);
-            if (lane + d < 32) t = agg_combine(t, o, vc);
-        }
-        if (lane == 0) s_warp[warp] = t;
-    }
-    __syncthreads();
-    if (tid == 0) {
-        Agg<NV> r = agg_identity<NV>();
-        for (int w = 0; w < WARPS; ++w)
-            if ((w + 1) * 32 * ITEMS - 1 >= from) r = agg_combine(r, s_warp[w], vc);
-        r.heads = tile_heads;
-        tile_agg[tile] = r;
-    }
-}
-
-// Each CTA reduces several tiles in turn: 512-row tiles are too short to
-// amortise a CTA's launch.
-template <int NK, int NV>
-__global__ void __launch_bounds__(kSegThreads) k_seg_tiles(SegArgs a, Agg<NV>* tile_agg, uint32_t tiles) {
-    __shared__ TileSmem<NV> sm;
-    for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-        seg_tile_body<NK, NV>(a, tile_agg, t, sm);
-        __syncthreads();  // shared memory is reused by the next tile
-    }
-}
-
-// The same tile aggregates with eight rows per thread: one CTA covers
-// kSubTiles consecutive 512-row tiles (two warps each), so the pass runs a
-// quarter as many CTAs with four times the loads in flight per thread.
+// Eight rows per thread: one CTA covers kSubTiles consecutive 512-row tiles
+// (two warps each).
 constexpr int kWideItems = 8;
 constexpr int kSubTiles = kSegThreads * kWideItems / kSegTile;  // 4
 constexpr int kWarpsPerSub = kSegThreads / 32 / kSubTiles;      // 2
@@ -613,584 +386,293 @@ __global__ void __launch_bounds__(kScanTiles) k_seg_scan2(const SegArgs a, Agg<N
     }
 }
 
-// ---- phase 3: scan each tile from its prefix and emit the groups -------------
-// A tile where every row starts a group (typical when most keys are
-// distinct) needs no scan: row r is group H + (r - first row), H = heads
-// before the tile, and the group ending at row r - 1 is emitted at row r as
-// everywhere else, so a row's own one-row record is written here when the
-// next row is in the tile (or r is the last row) and the tile's first row
-// emits the group carried in from earlier tiles.  Every column is written
-// by consecutive lanes.  Records are built with the same operations as the
-// scanning path, so results are bit-identical.
-// TPT threads cover the tile, RPT rows each (row tile_first + j * TPT + tt),
-// loaded BATCH rows at a time before they are stored.
-template <int NK, int NV, int TPT, int RPT, int BATCH>
-__device__ __forceinline__ void emit_single_rows(const SegArgs& a, const Agg<NV>* tile_prefix,
-                                                 const Agg<NV>* block_prefix, uint32_t tile, uint32_t H,
-                                                 const int* vc, const int* kw, int tt) {
-    static_assert(TPT * RPT == kSegTile && RPT % BATCH == 0, "tile layout");
-    const uint64_t n = a.n;
-    const uint64_t first = (uint64_t)tile * kSegTile;
-    if (tt == 0 && H > 0) {
-        const Agg<NV> P = agg_combine(block_prefix[tile / kScanTiles], tile_prefix[tile], vc);
-        emit_group<NV>(a, H - 1, P.cnt, P.w, vc);
-    }
-#pragma unroll
-    for (int j0 = 0; j0 < RPT; j0 += BATCH) {
-        // every load of the batch before its first store (outputs may not be
-        // assumed apart from inputs, so the compiler would not reorder them)
-        uint64_t kx[BATCH][NK];
-        uint64_t vx[BATCH][NV > 0 ? NV : 1];
-#pragma unroll
-        for (int j = 0; j < BATCH; ++j) {
-            const uint64_t r = first + (uint64_t)(j0 + j) * TPT + tt;
-#pragma unroll
-            for (int k = 0; k < NK; ++k) kx[j][k] = r < n ? load_raw(a.key[k].src, kw[k], r) : 0ull;
-#pragma unroll
-            for (int v = 0; v < NV; ++v) vx[j][v] = r < n ? load_val(a.val[v].src, a.val[v].dtype, r) : 0ull;
-        }
-#pragma unroll
-        for (int j = 0; j < BATCH; ++j) {
-            const uint32_t o = (uint32_t)(j0 + j) * TPT + (uint32_t)tt;
-            const uint64_t r = first + o;
-            if (r >= n) break;
-            const uint32_t g = H + o;
-#pragma unroll
-            for (int k = 0; k < NK; ++k)
-                if (a.key_out[k]) store_raw(a.key_out[k], kw[k], g, kx[j][k]);
-            if (a.group_start) a.group_start[g] = (uint32_t)r;
-            if (a.row_group) a.row_group[r] = g;
-            if (o + 1 < (uint32_t)kSegTile || r == n - 1) {
-                uint64_t w[NV > 0 ? NV : 1][4];
-#pragma unroll
-                for (int v = 0; v < NV; ++v) col_init(w[v], vx[j][v], vc[v]);
-                emit_group<NV>(a, g, 1, w, vc);
-            }
-            if (r == n - 1 && a.n_groups) *a.n_groups = g + 1;
-        }
-    }
-}
+// ---- phase 3: emit the groups of each CTA's rows ------------------------------
+// Heads before tile t are the exclusive prefix of the tile pass's head counts,
+// so a CTA knows the heads in its rows before it reads them (all but the last
+// CTA: the prefix past the last tile is not stored).
+//   * None: it writes nothing unless rows' groups are wanted (row_group) and
+//     returns -- a CTA writes the group that ends before each head in its
+//     rows, with the new group's key and first row; a group running through
+//     head-less rows is written where the next head is.  With few groups over
+//     many rows nearly every CTA returns, and its rows are not read a second
+//     time.
+//   * As many as rows (most keys distinct): row r is group H + r, written
+//     straight from its loads.
+// The CTA holding the last row writes the last group and the group count.
 
-// Tiles where nearly every row starts a group (few groups of two or more
-// rows): rows are striped over the TPT threads (row first + j * TPT + tt),
-// so that records of one-row groups go out with consecutive lanes at
-// (nearly) consecutive group ids; the head row of a longer group walks that
-// group's few rows itself.  A group is emitted by the tile holding its last
-// row: one that runs past the tile's end is left to the next tile, whose
-// prefix carries it.  hm[t] / hp[t]: head mask of the sub-tile's 8-row block
-// t (consecutive rows 8t .. 8t+7) and the number of heads in blocks before
-// it within its warp of blocks (32 blocks), wh[w]: heads in warp w's blocks.
-template <int NK, int NV, int TPT, int RPT>
-__device__ __forceinline__ void emit_mostly_single(const SegArgs& a, const Agg<NV>* tile_prefix,
-                                                   const Agg<NV>* block_prefix, uint32_t tile, uint32_t H,
-                                                   const uint32_t* hm, const uint32_t* hp, const uint32_t* wh,
-                                                   const int* vc, const int* kw, int tt) {
-    constexpr int B = 8;  // rows per head-mask block
-    static_assert(TPT * RPT == kSegTile && kSegTile / B <= TPT * RPT, "tile layout");
-    const uint64_t n = a.n;
-    const uint64_t first = (uint64_t)tile * kSegTile;
-    const uint32_t rows = (uint32_t)min((uint64_t)kSegTile, n - first);
-    // is tile row o a head? (o == rows: the row after the tile)
-    auto is_head = [&](uint32_t o) -> bool {
-        if (o >= rows) {
-            if (first + o >= n) return true;
-            bool d = false;
-#pragma unroll
-            for (int k = 0; k < NK; ++k)
-                d |= load_raw(a.key[k].src, kw[k], first + o) != load_raw(a.key[k].src, kw[k], first + o - 1);
-            return d;
-        }
-        return (hm[o / B] >> (o % B)) & 1u;
-    };
-    auto heads_before = [&](uint32_t o) -> uint32_t {  // heads among tile rows < o
-        const uint32_t t = o / B;
-        uint32_t c = hp[t] + __popc(hm[t] & ((1u << (o % B)) - 1u));
-        for (uint32_t w = 0; w < t / 32; ++w) c += wh[w];
-        return c;
-    };
-    // Aggregate of tile rows [o, end) up to the next head; returns the end.
-    auto walk = [&](uint32_t o, uint64_t (*w)[4], uint32_t& cnt) -> uint32_t {
-        uint32_t e = o;
-        while (e < rows && (e == o || !is_head(e))) {
-            const uint64_t r = first + e;
-#pragma unroll
-            for (int v = 0; v < NV; ++v) {
-                const uint64_t x = load_val(a.val[v].src, a.val[v].dtype, r);
-                if (cnt == 0) {
-                    col_init(w[v], x, vc[v]);
-                } else {
-                    uint64_t one[4];
-                    col_init(one, x, vc[v]);
-                    col_merge(w[v], one, vc[v]);
-                }
-            }
-            ++cnt;
-            ++e;
-        }
-        return e;
-    };
-    // the group carried in from earlier tiles (id H - 1): it ends before the
-    // first row if that is a head, else at the tile's first head after it
-    if (tt == 0 && H > 0) {
-        const Agg<NV> P = agg_combine(block_prefix[tile / kScanTiles], tile_prefix[tile], vc);
-        uint64_t w[NV > 0 ? NV : 1][4];
-#pragma unroll
-        for (int v = 0; v < NV; ++v)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) w[v][q] = P.w[v][q];
-        uint32_t cnt = P.cnt;
-        bool ends = true;
-        if (!is_head(0)) {
-            uint32_t e = 0;
-            while (e < rows && !is_head(e)) {
-                const uint64_t r = first + e;
-#pragma unroll
-                for (int v = 0; v < NV; ++v) {
-                    uint64_t one[4];
-                    col_init(one, load_val(a.val[v].src, a.val[v].dtype, r), vc[v]);
-                    col_merge(w[v], one, vc[v]);
-                }
-                ++cnt;
-                ++e;
-            }
-            ends = e < rows || first + e == n || is_head(e);
-        }
-        if (ends) emit_group<NV>(a, H - 1, cnt, w, vc);
-    }
-#pragma unroll 1
-    for (int j = 0; j < RPT; ++j) {
-        const uint32_t o = (uint32_t)j * TPT + (uint32_t)tt;
-        if (o >= rows) break;
-        const uint64_t r = first + o;
-        const bool h = is_head(o);
-        const uint32_t hb = heads_before(o);
-        const uint32_t grow = h ? H + hb : H + hb - 1;  // the group of row r
-        if (a.row_group) a.row_group[r] = grow;
-        if (r == n - 1 && a.n_groups) *a.n_groups = grow + 1;
-        if (!h) continue;
-        const uint32_t g = H + hb;
-#pragma unroll
-        for (int k = 0; k < NK; ++k)
-            if (a.key_out[k]) store_raw(a.key_out[k], kw[k], g, load_raw(a.key[k].src, kw[k], r));
-        if (a.group_start) a.group_start[g] = (uint32_t)r;
-        uint64_t w[NV > 0 ? NV : 1][4];
-        uint32_t cnt = 0;
-        const uint32_t e = walk(o, w, cnt);
-        // complete when the next head (or the last row) is inside this tile
-        if (e < rows || first + e == n || is_head(e)) emit_group<NV>(a, g, cnt, w, vc);
-    }
-}
-
-template <int NK, int NV>
-__device__ __forceinline__ void seg_emit_body(const SegArgs& a, const Agg<NV>* tile_prefix, const Agg<NV>* block_prefix,
-                                              uint32_t tile) {
-    constexpr int ITEMS = kSegItems;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint64_t n = a.n;
-    const uint64_t row0 = (uint64_t)tile * kSegTile + (uint64_t)tid * ITEMS;
-    Agg<NV>* s_warp = reinterpret_cast<Agg<NV>*>(seg_smem);  // two buffers of [1 + 8] (see below)
-    int vc[NV > 0 ? NV : 1], kw[NK];
-    seg_setup<NK, NV>(a, vc, kw);
-    // heads before the tile, loaded first so that its latency overlaps the key loads
-    const uint32_t H_tile = block_prefix[tile / kScanTiles].heads + tile_prefix[tile].heads;
-    const uint32_t hmask = row_heads<NK>(a, row0, lane, kw);
-    const uint32_t nvalid = row0 >= n ? 0u : (n - row0 >= (uint64_t)ITEMS ? (uint32_t)ITEMS : (uint32_t)(n - row0));
-    if (__syncthreads_and(hmask == (1u << nvalid) - 1u)) {
-        emit_single_rows<NK, NV, kSegThreads, kSegItems, kSegItems>(a, tile_prefix, block_prefix, tile, H_tile, vc,
-                                                                     kw, tid);
-        return;
-    }
-    const Agg<NV> t = fold_rows<NV>(a, row0, vc, hmask);
-    // Per warp: the aggregate of the lanes before each lane (lx) and the
-    // warp's total.  When every lane's first row starts a group (typical with
-    // many groups), no segment crosses into a lane, so a lane's carry is just
-    // the previous lane's trailing segment plus a count of heads: one shuffle
-    // of the aggregate and a 32-bit scan instead of a scan of aggregates.
-    Agg<NV> lx, wtot;
-    if (__all_sync(0xffffffffu, row0 >= n || (hmask & 1u))) {
-        const uint32_t h = __popc(hmask);
-        uint32_t ih = h;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t o = __shfl_up_sync(0xffffffffu, ih, d);
-            if (lane >= d) ih += o;
-        }
-        lx = agg_shfl_up(t, 1);  // previous lane's trailing segment
-        lx.heads = ih - h;
-        if (lane == 0) lx = agg_identity<NV>();
-        wtot = t;  // (read at lane 31) its trailing segment, and all heads
-        wtot.heads = ih;
-    } else {
-        Agg<NV> incl = t;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const Agg<NV> o = agg_shfl_up(incl, d);
-            if (lane >= d) incl = agg_combine(o, incl, vc);
-        }
-        lx = agg_shfl_up(incl, 1);
-        if (lane == 0) lx = agg_identity<NV>();
-        wtot = incl;
-    }
-    // [0] tile prefix, [1 + w] total of warp w; warp 0 scans these nine
-    // entries in shared memory (double-buffered, four steps) into each warp's
-    // exclusive prefix, so every thread then combines once
-    constexpr int WARPS = kSegThreads / 32;
-    if (lane == 31) s_warp[1 + warp] = wtot;
-    if (tid == 0) s_warp[0] = agg_combine(block_prefix[tile / kScanTiles], tile_prefix[tile], vc);
-    __syncthreads();
-    if (warp == 0) {
-        Agg<NV>* src = s_warp;
-        Agg<NV>* dst = s_warp + (WARPS + 1);
-#pragma unroll 1
-        for (int d = 1; d <= WARPS; d <<= 1) {
-            if (lane <= WARPS) dst[lane] = lane >= d ? agg_combine(src[lane - d], src[lane], vc) : src[lane];
-            __syncwarp();
-            Agg<NV>* t2 = src;
-            src = dst;
-            dst = t2;
-        }
-    }
-    __syncthreads();
-    const Agg<NV> pre = agg_combine(s_warp[warp], lx, vc);  // four steps: the result is back in s_warp
-
-    // A segment is complete when the next head (or the last row) is reached;
-    // the thread that reaches it produces the group's record.  The groups a
-    // warp completes, and the groups whose heads lie in its rows, have
-    // consecutive ids, so records and keys are staged in the warp's shared
-    // memory and every output column is then written by consecutive lanes.
-    using Stage = WarpStage<NK, NV, ITEMS>;
-    Stage& st = reinterpret_cast<Stage*>(seg_smem + stage_offset<NK, NV>())[warp];
-    const uint32_t H_w = __shfl_sync(0xffffffffu, pre.heads, 0);  // heads before the warp's first row
-    const uint32_t g0 = H_w > 0 ? H_w - 1 : 0;                     // first group the warp completes
-    uint32_t gid = pre.heads;
-    uint32_t cnt = pre.cnt;
+// The aggregate of some rows of one group: lanes or threads build it row by
+// row, a warp merges its lanes'.
+template <int NV>
+struct Fold {
+    uint32_t cnt = 0;
     uint64_t w[NV > 0 ? NV : 1][4];
+    __device__ __forceinline__ void row(const uint64_t* vals, uint32_t stride, const int* vc) {
 #pragma unroll
-    for (int v = 0; v < NV; ++v)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) w[v][q] = pre.w[v][q];
-    uint32_t rg[ITEMS];
-    uint32_t emitted = 0;
-#pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-        const uint64_t r = row0 + j;
-        rg[j] = 0;
-        if (r >= n) break;
-        uint64_t val[NV > 0 ? NV : 1];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) val[v] = load_val(a.val[v].src, a.val[v].dtype, r);
-        if ((hmask >> j) & 1u) {
-            if (gid > 0) {
-                st.put(gid - 1 - g0, cnt, w);
-                ++emitted;
-            }
-            ++gid;
-            const int ki = Stage::at(gid - 1 - H_w);
-#pragma unroll
-            for (int k = 0; k < NK; ++k) st.key[k][ki] = load_raw(a.key[k].src, kw[k], r);
-            st.start[ki] = (uint32_t)r;
-            cnt = 1;
-#pragma unroll
-            for (int v = 0; v < NV; ++v) col_init(w[v], val[v], vc[v]);
-        } else {
-            ++cnt;
-#pragma unroll
-            for (int v = 0; v < NV; ++v) {
+        for (int v = 0; v < NV; ++v) {
+            const uint64_t x = vals[v * stride];
+            if (cnt == 0) {
+                col_init(w[v], x, vc[v]);
+            } else {
                 uint64_t one[4];
-                col_init(one, val[v], vc[v]);
+                col_init(one, x, vc[v]);
                 col_merge(w[v], one, vc[v]);
             }
         }
-        rg[j] = gid - 1;
-        if (r == n - 1) {
-            st.put(gid - 1 - g0, cnt, w);
-            ++emitted;
-            if (a.n_groups) *a.n_groups = gid;
+        ++cnt;
+    }
+    __device__ __forceinline__ void merge(const Fold& o, const int* vc) {
+        if (o.cnt == 0) return;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            if (cnt == 0) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) w[v][q] = o.w[v][q];
+            } else {
+                col_merge(w[v], o.w[v], vc[v]);
+            }
+        }
+        cnt += o.cnt;
+    }
+    // afterwards each of `lanes` (a power of two) neighbouring lanes holds the sum of theirs
+    __device__ __forceinline__ void team(int lanes, const int* vc) {
+#pragma unroll 1
+        for (int d = 1; d < lanes; d <<= 1) {
+            Fold o;
+            o.cnt = __shfl_xor_sync(0xffffffffu, cnt, d);
+#pragma unroll
+            for (int v = 0; v < NV; ++v)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) o.w[v][q] = __shfl_xor_sync(0xffffffffu, w[v][q], d);
+            merge(o, vc);
         }
     }
-    if (a.row_group && row0 < n) {
-        if (row0 + ITEMS <= n && (reinterpret_cast<uintptr_t>(a.row_group + row0) & 7) == 0) {
-            *reinterpret_cast<uint2*>(a.row_group + row0) = make_uint2(rg[0], rg[1]);
-        } else {
-#pragma unroll
-            for (int j = 0; j < ITEMS; ++j)
-                if (row0 + j < n) a.row_group[row0 + j] = rg[j];
-        }
-    }
-    uint32_t E = emitted;
-    uint32_t K = __popc(hmask);
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-        E += __shfl_xor_sync(0xffffffffu, E, d);
-        K += __shfl_xor_sync(0xffffffffu, K, d);
-    }
-    __syncwarp();
-    for (uint32_t i = lane; i < E; i += 32) {
-        const int x = Stage::at(i);
-        uint64_t gw[NV > 0 ? NV : 1][4];
-#pragma unroll
-        for (int v = 0; v < NV; ++v)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) gw[v][q] = st.w[v][q][x];
-        emit_group<NV>(a, g0 + i, st.cnt[x], gw, vc);
-    }
-    for (uint32_t i = lane; i < K; i += 32) {
-        const int x = Stage::at(i);
-#pragma unroll
-        for (int k = 0; k < NK; ++k)
-            if (a.key_out[k]) store_raw(a.key_out[k], kw[k], H_w + i, st.key[k][x]);
-        if (a.group_start) a.group_start[H_w + i] = st.start[x];
-    }
-}
+};
 
-// Tiles t0 .. t1-1 write nothing in the emit pass when no segment head lies
-// in their rows and no row's group is wanted (row_group): a tile writes the
-// group that ends before each head in it (with the new group's key and first
-// row), and the group running through head-less tiles is written where the
-// next head is.  The tile holding the last row (which writes the last group
-// and the group count) is never quiet; nor is t1 past the last tile, whose
-// prefix is not stored.  Heads before tile t are the exclusive prefix of the
-// tile pass's head counts, so the heads in the range are H(t1) - H(t0).  With
-// few groups over many rows (a low-cardinality key) nearly every tile is
-// quiet, and its rows are not read a second time.
+constexpr int kEmitRows = kSubTiles * kSegTile;        // rows of a CTA
+constexpr int kEmitPer = kEmitRows / kSegThreads;      // rows per thread
+constexpr int kEmitWords = kEmitRows / 32;             // head-mask words
+constexpr uint32_t kThreadRows = 32, kTeamRows = 256;  // longest group one thread and eight lanes fold
+static_assert(kEmitWords == 64 && kEmitRows <= 65536, "two words per lane of a warp; rows in 16 bits");
+
+extern __shared__ __align__(16) unsigned char seg_smem[];
 template <int NV>
-__device__ __forceinline__ bool quiet_tiles(const SegArgs& a, const Agg<NV>* tile_prefix, const Agg<NV>* block_prefix,
-                                            uint32_t t0, uint32_t t1, uint32_t tiles) {
-    if (a.row_group || t1 >= tiles) return false;
-    const uint32_t h0 = block_prefix[t0 / kScanTiles].heads + tile_prefix[t0].heads;
-    const uint32_t h1 = block_prefix[t1 / kScanTiles].heads + tile_prefix[t1].heads;
-    return h1 == h0;
-}
+constexpr size_t emit_smem_bytes() { return (size_t)NV * kEmitRows * 8; }
 
-template <int NK, int NV>
-__global__ void __launch_bounds__(kSegThreads, (NV >= 3 ? 1 : (NV == 2 ? 4 : 3))) k_seg_emit(SegArgs a, const Agg<NV>* tile_prefix,
-                                                                          const Agg<NV>* block_prefix, uint32_t tiles) {
-    for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-        if (quiet_tiles(a, tile_prefix, block_prefix, t, t + 1, tiles)) continue;  // the same for the whole CTA
-        seg_emit_body<NK, NV>(a, tile_prefix, block_prefix, t);
-        __syncthreads();  // the warp totals and staging are reused by the next tile
-    }
-}
-
-// The emit pass with eight rows per thread: each 512-row tile is taken by
-// two warps (kSubTiles tiles per CTA, as in the reduce pass), so a warp scan
-// of aggregates and the cross-warp step are shared by eight rows instead of
-// two, and each row costs one merge in the final walk.  A thread's rows are
-// consecutive: its groups complete in order and are written as they
-// complete.  Tiles where every row starts a group take the one-row-record
-// path with coalesced writes.
+// A CTA takes four tiles: its rows' values go into shared memory, the heads
+// become a list of group starts, and then one thread folds and writes each
+// group of up to kThreadRows rows -- consecutive threads consecutive groups,
+// so every output column is written by full warps -- eight lanes each longer
+// group, and one warp each group past kTeamRows and the one running in from
+// earlier rows (whose part before the CTA is the tile prefix).  Where nearly every row starts a group (from
+// striped_min_heads of 512 rows) the threads go by rows instead of by groups.
+//
+// What bounds it: instructions.  A thread per eight rows that scanned
+// aggregates of 18 words across the warp and wrote each group where its rows
+// ended (a quarter of the lanes storing at a time) took 341 instructions per
+// row of a batch of short groups.  Per launch on one B200, that kernel ->
+// this one: 200M rows of 50M keys 4.76 -> 2.42 ms, 9M rows in groups of two
+// 0.32 -> 0.25 ms, 100M one-row groups of two keys 2.09 -> 1.80 ms (12.2 GB:
+// HBM-bound), a batch of 4,096 queries 1.26 -> 1.07 ms, 1M rows in groups of
+// 100 22.9 -> 15.1 us.
 template <int NK, int NV, int VCP = 0, int KWP = 0>
-__global__ void __launch_bounds__(kSegThreads, (NV >= 3 ? 1 : 3))
-    k_seg_emit_wide(SegArgs a, const Agg<NV>* tile_prefix, const Agg<NV>* block_prefix, uint32_t tiles) {
-    constexpr int ITEMS = kWideItems, WARPS = kSegThreads / 32;
-    __shared__ Agg<NV> s_wtot[WARPS];
-    __shared__ Agg<NV> s_pre[kSubTiles];
-    __shared__ uint32_t s_all[WARPS];
-    __shared__ uint32_t s_hm[kSegThreads];  // head mask of each thread's rows
-    __shared__ uint32_t s_hp[kSegThreads];  // heads before them in the warp
-    __shared__ uint32_t s_wh[WARPS];        // heads in each warp's rows
-    // tiles without a segment head write nothing (uniform over the CTA, so
-    // before any barrier)
-    if (quiet_tiles(a, tile_prefix, block_prefix, blockIdx.x * kSubTiles, (blockIdx.x + 1) * kSubTiles, tiles))
-        return;
+__global__ void __launch_bounds__(kSegThreads, (NV >= 3 ? 2 : 4))
+    k_seg_emit(SegArgs a, const Agg<NV>* tile_prefix, const Agg<NV>* block_prefix, uint32_t tiles) {
+    constexpr int R = kEmitPer, B = 4;  // rows per thread, loaded B at a time
+    uint64_t* vals = reinterpret_cast<uint64_t*>(seg_smem);  // [NV][kEmitRows]
+    __shared__ uint32_t s_word[kEmitWords], s_pre[kEmitWords + 1];
+    __shared__ uint16_t s_pos[kEmitRows + 1];  // first row of each group that starts here
+    __shared__ uint16_t s_long[kEmitRows / (kThreadRows + 1) + 1];  // the longer groups
+    __shared__ uint32_t s_nlong;
+    const uint32_t t0 = blockIdx.x * kSubTiles, t1 = t0 + kSubTiles;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int sub = warp / kWarpsPerSub, wsub = warp - sub * kWarpsPerSub;
-    const uint32_t tile = blockIdx.x * kSubTiles + sub;
-    const bool tvalid = tile < tiles;
-    const int sub_tid = tid - sub * kWarpsPerSub * 32;
-    const uint64_t n = a.n;
-    const uint64_t row0 = (uint64_t)tile * kSegTile + (uint64_t)sub_tid * ITEMS;
+    const uint64_t n = a.n, base = (uint64_t)t0 * kSegTile;
+    const uint32_t rows = (uint32_t)min((uint64_t)kEmitRows, n - base);
+    const bool table_end = base + rows == n;
     int vc[NV > 0 ? NV : 1], kw[NK];
     seg_setup<NK, NV>(a, vc, kw);
     fix_classes<NV, VCP>(vc);
     fix_widths<NK, KWP>(kw);
-    // heads before the tile, loaded first so that its latency overlaps the key loads
-    const uint32_t H_tile = tvalid ? block_prefix[tile / kScanTiles].heads + tile_prefix[tile].heads : 0u;
+    // groups that start before the CTA's rows, and in them where that is known
+    const uint32_t H = block_prefix[t0 / kScanTiles].heads + tile_prefix[t0].heads;
+    const uint32_t known = t1 < tiles ? block_prefix[t1 / kScanTiles].heads + tile_prefix[t1].heads - H : ~0u;
+    if (known == 0 && !a.row_group) return;  // the same for the whole CTA
+    // the group running in from earlier rows ends at the CTA's row e, the first
+    // head: one warp adds the rows from e's own tile on to that tile's prefix
+    auto carried = [&](uint32_t e) {
+        const uint32_t sub = (e ? e - 1 : 0u) / kSegTile;
+        Fold<NV> f;
+#pragma unroll 1
+        for (uint32_t r = sub * kSegTile + lane; r < e; r += 32) f.row(vals + r, kEmitRows, vc);
+        if (e) f.team(32, vc);
+        if (lane == 0) {
+            const Agg<NV> P = agg_combine(block_prefix[(t0 + sub) / kScanTiles], tile_prefix[t0 + sub], vc);
+            Fold<NV> c;
+            c.cnt = P.cnt;
+#pragma unroll
+            for (int v = 0; v < NV; ++v)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) c.w[v][q] = P.w[v][q];
+            c.merge(f, vc);
+            emit_group<NV>(a, H - 1, c.cnt, c.w, vc);
+        }
+    };
+    if (known == (uint32_t)kEmitRows) {
+        if (warp == 0 && H > 0) carried(0);
+#pragma unroll
+        for (int j0 = 0; j0 < R; j0 += B) {
+            // every load of the batch before its first store (outputs may not
+            // be assumed apart from inputs, so the compiler would not reorder them)
+            uint64_t key[B][NK], x[B][NV > 0 ? NV : 1];
+#pragma unroll
+            for (int j = 0; j < B; ++j) {
+                const uint64_t r = base + (uint32_t)(j0 + j) * kSegThreads + tid;
+#pragma unroll
+                for (int k = 0; k < NK; ++k) key[j][k] = load_raw(a.key[k].src, kw[k], r);
+#pragma unroll
+                for (int v = 0; v < NV; ++v) x[j][v] = load_val(a.val[v].src, a.val[v].dtype, r);
+            }
+#pragma unroll
+            for (int j = 0; j < B; ++j) {
+                const uint32_t o = (uint32_t)(j0 + j) * kSegThreads + tid, g = H + o;
+#pragma unroll
+                for (int k = 0; k < NK; ++k)
+                    if (a.key_out[k]) store_raw(a.key_out[k], kw[k], g, key[j][k]);
+                if (a.group_start) a.group_start[g] = (uint32_t)(base + o);
+                if (a.row_group) a.row_group[base + o] = g;
+                if (o + 1 == (uint32_t)kEmitRows) break;  // may go on: left to the next CTA (never the table's last row)
+                uint64_t w[NV > 0 ? NV : 1][4];
+#pragma unroll
+                for (int v = 0; v < NV; ++v) col_init(w[v], x[j][v], vc[v]);
+                emit_group<NV>(a, g, 1, w, vc);
+            }
+        }
+        return;
+    }
 
-    uint32_t hmask = 0;
-    {
-        uint64_t key[ITEMS][NK];
+    if (tid == 0) s_nlong = 0;
+    uint32_t mine = 0;  // bit j: row j * kSegThreads + tid starts a group
 #pragma unroll
-        for (int k = 0; k < NK; ++k) load_rows<ITEMS>(a.key[k].src, kw[k], row0, n, key, k);
-        uint64_t prev[NK];
+    for (int j0 = 0; j0 < R; j0 += B) {
+        uint64_t key[B][NK], before[B][NK], x[B][NV > 0 ? NV : 1];
 #pragma unroll
-        for (int k = 0; k < NK; ++k) prev[k] = __shfl_up_sync(0xffffffffu, key[ITEMS - 1][k], 1);
-        if (lane == 0 && row0 > 0 && row0 < n) {
+        for (int j = 0; j < B; ++j) {
+            const uint32_t r = (uint32_t)(j0 + j) * kSegThreads + tid;
+            const bool ok = r < rows;
 #pragma unroll
-            for (int k = 0; k < NK; ++k) prev[k] = load_raw(a.key[k].src, kw[k], row0 - 1);
+            for (int k = 0; k < NK; ++k) {
+                key[j][k] = ok ? load_raw(a.key[k].src, kw[k], base + r) : 0ull;
+                before[j][k] = ok && lane == 0 && base + r > 0 ? load_raw(a.key[k].src, kw[k], base + r - 1) : 0ull;
+            }
+#pragma unroll
+            for (int v = 0; v < NV; ++v) x[j][v] = ok ? load_val(a.val[v].src, a.val[v].dtype, base + r) : 0ull;
         }
 #pragma unroll
-        for (int j = 0; j < ITEMS; ++j) {
-            const uint64_t r = row0 + j;
-            bool h = (r == 0);
+        for (int j = 0; j < B; ++j) {
+            const uint32_t r = (uint32_t)(j0 + j) * kSegThreads + tid;
+            bool h = base + r == 0;
 #pragma unroll
-            for (int k = 0; k < NK; ++k) h |= (j == 0 ? prev[k] : key[j - 1][k]) != key[j][k];
-            if (r < n && h) hmask |= 1u << j;
+            for (int k = 0; k < NK; ++k) {
+                const uint64_t up = __shfl_up_sync(0xffffffffu, key[j][k], 1);
+                h |= (lane ? up : before[j][k]) != key[j][k];
+            }
+            h = h && r < rows;
+            const uint32_t word = __ballot_sync(0xffffffffu, h);
+            if (lane == 0) s_word[(j0 + j) * (kSegThreads / 32) + warp] = word;
+            mine |= h ? 1u << (j0 + j) : 0u;
+#pragma unroll
+            for (int v = 0; v < NV; ++v) vals[v * kEmitRows + r] = x[j][v];
         }
     }
-    const uint32_t nvalid = row0 >= n ? 0u : (n - row0 >= (uint64_t)ITEMS ? (uint32_t)ITEMS : (uint32_t)(n - row0));
-    const bool wall = __all_sync(0xffffffffu, hmask == (1u << nvalid) - 1u);
-    if (lane == 0) s_all[warp] = wall ? 1u : 0u;
-    {
-        const uint32_t h = __popc(hmask);
-        uint32_t ih = h;
+    __syncthreads();
+    if (warp == 0) {  // heads before each word
+        const uint32_t c0 = __popc(s_word[2 * lane]), c1 = __popc(s_word[2 * lane + 1]);
+        uint32_t incl = c0 + c1;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t o = __shfl_up_sync(0xffffffffu, ih, d);
-            if (lane >= d) ih += o;
+            const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += t;
         }
-        s_hm[tid] = hmask;
-        s_hp[tid] = ih - h;
-        if (lane == 31) s_wh[warp] = ih;
+        s_pre[2 * lane] = incl - c0 - c1;
+        s_pre[2 * lane + 1] = incl - c1;
+        if (lane == 31) s_pre[kEmitWords] = incl;
     }
     __syncthreads();
-    bool sub_all = true;
-    uint32_t sub_heads = 0;
+    const uint32_t heads = s_pre[kEmitWords];
+    const uint32_t lt = lanemask_lt();
+    auto index_of = [&](int j) -> uint32_t {  // groups that start here before row j * kSegThreads + tid
+        const int w = j * (kSegThreads / 32) + warp;
+        return s_pre[w] + __popc(s_word[w] & lt);
+    };
+    if (a.row_group) {
 #pragma unroll
-    for (int w = 0; w < kWarpsPerSub; ++w) {
-        sub_all = sub_all && s_all[sub * kWarpsPerSub + w] != 0u;
-        sub_heads += s_wh[sub * kWarpsPerSub + w];
+        for (int j = 0; j < R; ++j) {
+            const uint32_t r = (uint32_t)j * kSegThreads + tid;
+            if (r < rows) a.row_group[base + r] = H + index_of(j) + ((mine >> j) & 1u) - 1u;
+        }
     }
-    // many rows start a group (by default at most 32 rows continue one): the
-    // striped path
+    if (table_end && tid == 0 && a.n_groups) *a.n_groups = H + heads;
+#pragma unroll
+    for (int j = 0; j < R; ++j)
+        if ((mine >> j) & 1u) s_pos[index_of(j)] = (uint16_t)(j * kSegThreads + tid);
+    if (tid == 0) s_pos[heads] = (uint16_t)rows;
+    __syncthreads();
+    // the last group that starts here is complete only at the table's end
+    const uint32_t whole = table_end ? heads : (heads ? heads - 1 : 0);
+    auto group = [&](uint32_t k) {
+        const uint32_t b = s_pos[k], e = s_pos[k + 1];
+#pragma unroll
+        for (int q = 0; q < NK; ++q)
+            if (a.key_out[q]) store_raw(a.key_out[q], kw[q], H + k, load_raw(a.key[q].src, kw[q], base + b));
+        if (a.group_start) a.group_start[H + k] = (uint32_t)(base + b);
+        if (k >= whole) return;
+        if (e - b > kThreadRows) {  // left to a team below
+            s_long[atomicAdd(&s_nlong, 1u)] = (uint16_t)k;
+            return;
+        }
+        Fold<NV> f;
+#pragma unroll 1
+        for (uint32_t r = b; r < e; ++r) f.row(vals + r, kEmitRows, vc);
+        emit_group<NV>(a, H + k, f.cnt, f.w, vc);
+    };
     const uint32_t min_heads = a.striped_min_heads ? a.striped_min_heads : kStripedMinHeads;
-    const bool sub_most = !sub_all && sub_heads >= min_heads;
-
-    Agg<NV> lx = agg_identity<NV>();
-    if (!sub_all && !sub_most) {
-        // this thread's trailing segment: rows from its last head (all rows
-        // when it has none).  Rows are consumed from the front of a shift
-        // register, so the loop stays rolled (one copy of the merge code)
-        // while the values stay in registers.
-        uint64_t val[ITEMS][NV > 0 ? NV : 1];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) load_vals<ITEMS>(a.val[v].src, a.val[v].dtype, row0, n, val, v);
-        const int from = hmask ? 31 - __clz(hmask) : 0;
-        const int upto = (int)nvalid;
-        Agg<NV> t = agg_identity<NV>();
-        t.heads = __popc(hmask);
+    if (heads >= min_heads * (uint32_t)kSubTiles) {
 #pragma unroll 1
-        for (int j = 0; j < upto; ++j) {
-            if (j >= from) {
-                if (t.cnt == 0) {
-#pragma unroll
-                    for (int v = 0; v < NV; ++v) col_init(t.w[v], val[0][v], vc[v]);
-                } else {
-#pragma unroll
-                    for (int v = 0; v < NV; ++v) {
-                        uint64_t one[4];
-                        col_init(one, val[0][v], vc[v]);
-                        col_merge(t.w[v], one, vc[v]);
-                    }
-                }
-                t.cnt++;
-            }
-#pragma unroll
-            for (int i = 0; i + 1 < ITEMS; ++i)
-#pragma unroll
-                for (int v = 0; v < NV; ++v) val[i][v] = val[i + 1][v];
-        }
-        // per warp: the aggregate of the lanes before each lane, and the total
-        Agg<NV> wtot;
-        if (__all_sync(0xffffffffu, row0 >= n || (hmask & 1u))) {
-            // no segment crosses into a lane: carry = previous lane's trailing
-            // segment, plus a count of heads
-            const uint32_t h = __popc(hmask);
-            uint32_t ih = h;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const uint32_t o = __shfl_up_sync(0xffffffffu, ih, d);
-                if (lane >= d) ih += o;
-            }
-            lx = agg_shfl_up(t, 1);
-            lx.heads = ih - h;
-            if (lane == 0) lx = agg_identity<NV>();
-            wtot = t;
-            wtot.heads = ih;
-        } else {
-            Agg<NV> incl = t;
+        for (int j = 0; j < R; ++j)
+            if ((mine >> j) & 1u) group(index_of(j));
+    } else {
 #pragma unroll 1
-            for (int d = 1; d < 32; d <<= 1) {
-                const Agg<NV> o = agg_shfl_up(incl, d);
-                if (lane >= d) incl = agg_combine(o, incl, vc);
-            }
-            lx = agg_shfl_up(incl, 1);
-            if (lane == 0) lx = agg_identity<NV>();
-            wtot = incl;
-        }
-        if (lane == 31) s_wtot[warp] = wtot;
-        if (wsub == 0 && lane == 0 && tvalid)
-            s_pre[sub] = agg_combine(block_prefix[tile / kScanTiles], tile_prefix[tile], vc);
+        for (uint32_t k = tid; k < heads; k += kSegThreads) group(k);
     }
-    __syncthreads();
-
-    if (sub_all) {
-        if (tvalid)
-            emit_single_rows<NK, NV, kWarpsPerSub * 32, ITEMS, ITEMS / 2>(a, tile_prefix, block_prefix, tile, H_tile,
-                                                                          vc, kw, sub_tid);
-        return;
-    }
-    if (sub_most) {
-        if (tvalid) {
-            const int base = sub * kWarpsPerSub * 32;
-            emit_mostly_single<NK, NV, kWarpsPerSub * 32, ITEMS>(a, tile_prefix, block_prefix, tile, H_tile,
-                                                                s_hm + base, s_hp + base, s_wh + sub * kWarpsPerSub,
-                                                                vc, kw, sub_tid);
-        }
-        return;
-    }
-    if (row0 >= n) return;
-    Agg<NV> pre = s_pre[sub];
-#pragma unroll
-    for (int w = 0; w < kWarpsPerSub; ++w)
-        if (w < wsub) pre = agg_combine(pre, s_wtot[sub * kWarpsPerSub + w], vc);
-    pre = agg_combine(pre, lx, vc);
-
-    // walk this thread's rows (rolled; each row's values read again, from L1
-    // after the fold above brought them in): a head completes the group
-    // before it.  Rows after the last head belong to a group that ends in a
-    // later thread, so the walk stops at the last head unless the rows' groups
-    // are wanted (row_group) or the thread holds the table's last row.
-    uint32_t gid = pre.heads;
-    uint32_t cnt = pre.cnt;
-    uint64_t w[NV > 0 ? NV : 1][4];
-#pragma unroll
-    for (int v = 0; v < NV; ++v)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) w[v][q] = pre.w[v][q];
-    const bool holds_last = row0 + nvalid == n;
-    const int upto = (a.row_group || holds_last) ? (int)nvalid : (hmask ? 32 - __clz(hmask) : 0);
+    // groups past one thread's rows, if there can be one: eight lanes or a warp each
+    if (rows - heads >= kThreadRows) {
+        __syncthreads();
+        const uint32_t nlong = s_nlong;
 #pragma unroll 1
-    for (int j = 0; j < upto; ++j) {
-        const uint64_t r = row0 + j;
-        uint64_t x[NV > 0 ? NV : 1];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) x[v] = load_val(a.val[v].src, a.val[v].dtype, r);
-        if ((hmask >> j) & 1u) {
-            if (gid > 0) emit_group<NV>(a, gid - 1, cnt, w, vc);
-#pragma unroll
-            for (int k = 0; k < NK; ++k)
-                if (a.key_out[k]) store_raw(a.key_out[k], kw[k], gid, load_raw(a.key[k].src, kw[k], r));
-            if (a.group_start) a.group_start[gid] = (uint32_t)r;
-            ++gid;
-            cnt = 1;
-#pragma unroll
-            for (int v = 0; v < NV; ++v) col_init(w[v], x[v], vc[v]);
-        } else {
-            ++cnt;
-#pragma unroll
-            for (int v = 0; v < NV; ++v) {
-                uint64_t one[4];
-                col_init(one, x[v], vc[v]);
-                col_merge(w[v], one, vc[v]);
+        for (uint32_t i0 = warp * 4; i0 < nlong; i0 += kSegThreads / 8) {
+            const uint32_t i = i0 + (lane >> 3);
+            const uint32_t k = i < nlong ? s_long[i] : 0;
+            const uint32_t b = s_pos[k], e = s_pos[k + 1];
+            const bool here = i < nlong && e - b <= kTeamRows;
+            Fold<NV> f;
+            if (here) {
+#pragma unroll 1
+                for (uint32_t r = b + (lane & 7); r < e; r += 8) f.row(vals + r, kEmitRows, vc);
             }
+            f.team(8, vc);
+            if (here && (lane & 7) == 0) emit_group<NV>(a, H + k, f.cnt, f.w, vc);
         }
-        if (a.row_group) a.row_group[r] = gid - 1;
+#pragma unroll 1
+        for (uint32_t i = warp; i < nlong; i += kSegThreads / 32) {
+            const uint32_t k = s_long[i], b = s_pos[k], e = s_pos[k + 1];
+            if (e - b <= kTeamRows) continue;
+            Fold<NV> f;
+#pragma unroll 1
+            for (uint32_t r = b + lane; r < e; r += 32) f.row(vals + r, kEmitRows, vc);
+            f.team(32, vc);
+            if (lane == 0) emit_group<NV>(a, H + k, f.cnt, f.w, vc);
+        }
     }
-    if (holds_last) {  // this thread holds the last row: its group ends there
-        emit_group<NV>(a, gid - 1, cnt, w, vc);
-        if (a.n_groups) *a.n_groups = gid;
-    }
+    if (warp == kSegThreads / 32 - 1 && H > 0 && (heads > 0 || table_end)) carried(s_pos[0]);  // (no head: rows)
 }
 
 template <int NK, int NV>
@@ -1199,7 +681,6 @@ cudaError_t seg_run(const SegArgs& a, unsigned char* aggs, uint32_t tiles, cudaS
     const uint32_t blocks = (tiles + kScanTiles - 1) / kScanTiles;
     Agg<NV>* bt = ta + tiles;
     if (prof) prof->begin(KC_SEGREDUCE, s);
-    const uint32_t grid = (tiles + kSegTilesPerCta - 1) / kSegTilesPerCta;
     // the float + signed-integer value pair with two keys of fixed widths
     // (8+4, 4+8, 4+4 bytes) gets fully specialised kernels
     const bool fixed = NV == 2 && value_class_pattern(a) == 1;
@@ -1234,40 +715,27 @@ cudaError_t seg_run(const SegArgs& a, unsigned char* aggs, uint32_t tiles, cudaS
     if (prof) prof->end(KC_SEGSCAN, s);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (prof) prof->begin(KC_SEGEMIT, s);
-    if constexpr (NV <= 2)
-    {
-        bool launched_emit = false;
-        if constexpr (NK == 2 && NV == 2) {
-            launched_emit = true;
-            if (kwp == 0x48)
-                k_seg_emit_wide<NK, NV, 1, 0x48><<<wide_grid, kSegThreads, 0, s>>>(a, ta, bt, tiles);
-            else if (kwp == 0x84)
-                k_seg_emit_wide<NK, NV, 1, 0x84><<<wide_grid, kSegThreads, 0, s>>>(a, ta, bt, tiles);
-            else if (kwp == 0x44)
-                k_seg_emit_wide<NK, NV, 1, 0x44><<<wide_grid, kSegThreads, 0, s>>>(a, ta, bt, tiles);
-            else
-                launched_emit = false;
-        }
-        if (!launched_emit) {
-            if constexpr (NV == 2) {
-                if (fixed) k_seg_emit_wide<NK, NV, 1><<<wide_grid, kSegThreads, 0, s>>>(a, ta, bt, tiles);
-                else k_seg_emit_wide<NK, NV, 0><<<wide_grid, kSegThreads, 0, s>>>(a, ta, bt, tiles);
-            } else {
-                k_seg_emit_wide<NK, NV, 0><<<wide_grid, kSegThreads, 0, s>>>(a, ta, bt, tiles);
-            }
-        }
+    constexpr size_t smem = emit_smem_bytes<NV>();
+    auto emit = k_seg_emit<NK, NV, 0>;
+    if constexpr (NV == 2) {
+        if (fixed) emit = k_seg_emit<NK, NV, 1>;
     }
-    else
-        k_seg_emit<NK, NV><<<grid, kSegThreads, emit_smem_bytes<NK, NV>(), s>>>(a, ta, bt, tiles);
+    if constexpr (NK == 2 && NV == 2) {
+        if (kwp == 0x48) emit = k_seg_emit<NK, NV, 1, 0x48>;
+        else if (kwp == 0x84) emit = k_seg_emit<NK, NV, 1, 0x84>;
+        else if (kwp == 0x44) emit = k_seg_emit<NK, NV, 1, 0x44>;
+    }
+    emit<<<wide_grid, kSegThreads, smem, s>>>(a, ta, bt, tiles);
     if (prof) prof->end(KC_SEGEMIT, s);
     return cudaGetLastError();
 }
 
+// Only three and four value columns need more than 48 KB (none of the
+// specialised instances does).
 template <int NK, int NV>
 cudaError_t seg_attr() {
-    constexpr size_t smem = emit_smem_bytes<NK, NV>();
-    static_assert(smem <= 227 * 1024, "group-by shared memory exceeds the per-CTA limit");
-    return cudaFuncSetAttribute(k_seg_emit<NK, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return cudaFuncSetAttribute(k_seg_emit<NK, NV, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)emit_smem_bytes<NV>());
 }
 
 template <int NK>
