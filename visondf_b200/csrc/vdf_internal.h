@@ -150,6 +150,9 @@ struct PassArgs {
     // word: 0 MSD-first passes, 1 LSD passes, 2 done by the dictionary pass)
     const uint32_t* run_flag;
     uint32_t run_when;
+    // ... and, with run_flag2 set, only when *run_flag2 == run_when2
+    const uint32_t* run_flag2 = nullptr;
+    uint32_t run_when2 = 0;
     // dictionary pass: the digit of a key is its rank among the sort's
     // distinct keys, looked up in this table
     const DictLut* dict_lut = nullptr;
@@ -208,11 +211,17 @@ struct SortPlan {
     // device decides, no host round trip).
     bool msd;
     int msd_passes;
+    // Two-pass plans of 8-byte keys take a third, lower top digit where the
+    // digits' histograms tell that two would leave buckets too large for the
+    // chunks (clustered keys: doubles around 1 share their exponents); a device
+    // word (off_msd_deep) says so, and the pass over that digit runs only then.
+    bool msd_deep;
+    int msd_digits;            // top digits with histograms: msd_passes, or one more
     int msd_lo_bits;           // key 0 bits ranked directly in runs (below the shared-memory passes)
     uint32_t msd_cap;          // rows a chunk may hold (kMsdCap or kMsdWideCap)
     uint32_t msd_chunk_rows;   // nominal rows per chunk
     uint32_t msd_chunks;       // ceil(n / msd_chunk_rows)
-    size_t off_msd_hist, off_msd_offs, off_msd_flag, off_chunks;
+    size_t off_msd_hist, off_msd_offs, off_msd_flag, off_msd_deep, off_chunks;
     // dictionary plan: a one-key sort whose key takes at most kDictMax
     // distinct values is one stable pass over each key's rank; the values
     // are collected on the device first, and with more of them the MSD-first
@@ -251,6 +260,7 @@ struct MsdChunkArgs {
     uint32_t chunk_rows, nchunks, pshift;
     uint32_t* chunk_start;  // [nchunks + 1]
     uint32_t* flag;
+    const uint32_t* deep = nullptr;  // non-null and set: the rows are sorted by eight more bits
     // segmented sorts: per-chunk descriptors, and a failure flag per segment
     const MsdSegChunk* seg_chunks = nullptr;
     uint32_t* seg_flag = nullptr;
@@ -264,6 +274,7 @@ struct MsdLocalArgs {
     int sec_dtype, dtype, invert, reverse;
     uint32_t lo_bits;        // key 0 bits below the shared-memory passes
     uint32_t pshift;         // key >> pshift: the bits the rows are sorted by (segmented: per chunk)
+    const uint32_t* deep;    // non-null and set: eight more bits
     uint32_t* flag;
     uint32_t* err;
     void* keys_out;          // raw sorted key 0 (may be null)
@@ -274,7 +285,9 @@ struct MsdLocalArgs {
     uint32_t* seg_flag = nullptr;
 };
 cudaError_t msd_hist(const MsdHistArgs& a, int width, cudaStream_t s);
-cudaError_t msd_scan(const uint32_t* hist, uint32_t* offs, int ndig, uint32_t cap, uint32_t* flag, cudaStream_t s);
+// deep (may be null): the lowest digit is optional, *deep is set when it is taken.
+cudaError_t msd_scan(const MsdHistArgs& a, int width, uint32_t* offs, uint32_t cap, uint32_t* flag, uint32_t* deep,
+                     cudaStream_t s);
 cudaError_t msd_chunks(const MsdChunkArgs& a, int width, cudaStream_t s, uint32_t cap = kMsdCap);
 cudaError_t msd_local(const MsdLocalArgs& a, int width, uint32_t nchunks, int match, cudaStream_t s,
                       uint32_t cap = kMsdCap);

@@ -324,6 +324,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_onesweep(PassArgs a) {
     // A conditional pass not taken returns before touching anything; the
     // flag was written by an earlier launch, so every thread reads the same.
     if (a.run_flag && *a.run_flag != a.run_when) return;
+    if (a.run_flag2 && *a.run_flag2 != a.run_when2) return;
     if constexpr (DICT) {  // the lookup table, used after the first barrier below
         for (uint32_t i = threadIdx.x; i < kDictLutSlots; i += THREADS) {
             dlk[i] = a.dict_lut->key[i];
@@ -1045,7 +1046,9 @@ SortPlan make_sort_plan(uint64_t n, const int32_t* dtypes, int nkeys, const Sort
     size_t off = 0;
     const size_t A = 256;
     const size_t status_bytes = (size_t)max_tiles * p.max_radix * 4;
-    const int msd_p = p.msd ? p.msd_passes : 0;
+    p.msd_deep = p.msd && p.msd_passes == 2 && p.width[0] == 8;
+    const int msd_p = p.msd ? p.msd_passes + (p.msd_deep ? 1 : 0) : 0;
+    p.msd_digits = msd_p;
     p.off_keys[0] = off; off = align_up(off + n * (size_t)maxw, A);
     p.off_keys[1] = off; off = align_up(off + n * (size_t)maxw, A);
     p.off_vals[0] = off; off = align_up(off + n * 4, A);
@@ -1072,7 +1075,8 @@ SortPlan make_sort_plan(uint64_t n, const int32_t* dtypes, int nkeys, const Sort
     if (p.msd || p.dict) {
         p.off_status[1] = off; off = align_up(off + status_bytes, A);
         if (p.msd) { p.off_msd_hist = off; off = align_up(off + (size_t)msd_p * 256 * 4, A); }
-        p.off_msd_flag = off; off = align_up(off + 4, A);
+        p.off_msd_flag = off;
+        p.off_msd_deep = off + 4; off = align_up(off + 8, A);
         if (p.dict) {
             p.off_dict_table = off; off = align_up(off + sizeof(DictSlot) * kDictSlots, A);
             p.off_dict_words = off; off = align_up(off + 16, A);
@@ -1090,7 +1094,7 @@ int sort_launches(const SortPlan& p) {
     // histogram + scan + passes, plus for the MSD plan its histogram, scan,
     // passes, chunk search and shared-memory finish (the LSD kernels are
     // launched in either case and return at once when not needed)
-    return 2 + p.total_passes + (p.msd ? 4 + p.msd_passes : 0) + (p.dict ? 3 : 0);
+    return 2 + p.total_passes + (p.msd ? 4 + p.msd_passes + (p.msd_deep ? 2 : 0) : 0) + (p.dict ? 3 : 0);
 }
 
 namespace {
@@ -1235,11 +1239,12 @@ cudaError_t run_msd(const SortPlan& p, const void* const* key_cols, int order, u
     const int w = p.width[0];
     const int P = p.msd_passes;
     const int ndigits = w;  // 8-bit digits
-    const int first = ndigits - P;
+    const int D = p.msd_digits, first = ndigits - D;
     cudaError_t e;
     uint32_t* mhist = reinterpret_cast<uint32_t*>(ws + p.off_msd_hist);
     uint32_t* moffs = reinterpret_cast<uint32_t*>(ws + p.off_msd_offs);
     uint32_t* flag = reinterpret_cast<uint32_t*>(ws + p.off_msd_flag);
+    uint32_t* deep = p.msd_deep ? reinterpret_cast<uint32_t*>(ws + p.off_msd_deep) : nullptr;
     uint32_t* counters = reinterpret_cast<uint32_t*>(ws + p.off_counters);
     uint32_t* status[2] = {reinterpret_cast<uint32_t*>(ws + p.off_status[0]),
                            reinterpret_cast<uint32_t*>(ws + p.off_status[1])};
@@ -1248,19 +1253,24 @@ cudaError_t run_msd(const SortPlan& p, const void* const* key_cols, int order, u
                          reinterpret_cast<uint32_t*>(ws + p.off_vals[1])};
     const bool invert = (order == 1);
 
-    MsdHistArgs mh{key_cols[0], p.dtype[0], invert ? 1 : 0, first, P, n, mhist, flag};
+    MsdHistArgs mh{key_cols[0], p.dtype[0], invert ? 1 : 0, first, D, n, mhist, flag};
     if (prof) prof->begin(KC_HIST, s);
     e = msd_hist(mh, w, s);
     if (prof) prof->end(KC_HIST, s);
     if (e != cudaSuccess) return e;
     if (prof) prof->begin(KC_SCAN, s);
-    e = msd_scan(mhist, moffs, P, p.msd_cap, flag, s);
+    e = msd_scan(mh, w, moffs, p.msd_cap, flag, deep, s);
     if (prof) prof->end(KC_SCAN, s);
     if (e != cudaSuccess) return e;
 
     const PassVariant& var = variant_for(p.tuning, w);
     const uint32_t tiles = (uint32_t)((n + var.threads * var.items - 1) / (var.threads * var.items));
-    for (int q = 0; q < P; ++q) {
+    // Pass q sorts by digit first + q, from buffer q - 1 to buffer q.  With an
+    // optional lowest digit, pass 0 runs only when it is taken, and pass 1 is
+    // launched twice: from the rows themselves when it is not, from pass 0's
+    // buffer when it is.  (The look-back status and tile counter of a pass not
+    // taken stay clear.)
+    auto pass = [&](int q, bool from_rows, const uint32_t* when, uint32_t is) -> cudaError_t {
         PassArgs a{};
         a.n = n;
         a.shift = (uint32_t)(8 * (first + q));
@@ -1276,31 +1286,37 @@ cudaError_t run_msd(const SortPlan& p, const void* const* key_cols, int order, u
         a.err = err;
         a.run_flag = flag;
         a.run_when = 0;
+        a.run_flag2 = when;
+        a.run_when2 = is;
         a.spin_limit = p.tuning.spin_limit;
-        a.stall_tile = q == 0 ? p.tuning.stall_tile : 0xffffffffu;
-        int mode;
-        if (q == 0) {
-            mode = perm_in ? IN_GATHER : IN_RAW;
-            a.keys_in = key_cols[0];
-            a.vals_in = perm_in;
-        } else {
-            mode = IN_BUF;
-            a.keys_in = kbuf[(q - 1) & 1];
-            a.vals_in = vbuf[(q - 1) & 1];
-        }
+        a.stall_tile = from_rows ? p.tuning.stall_tile : 0xffffffffu;
+        const int mode = !from_rows ? IN_BUF : perm_in ? IN_GATHER : IN_RAW;
+        a.keys_in = from_rows ? key_cols[0] : kbuf[(q - 1) & 1];
+        a.vals_in = from_rows ? perm_in : vbuf[(q - 1) & 1];
         a.keys_out = kbuf[q & 1];
         a.vals_out = vbuf[q & 1];
         a.ntiles = tiles;
-        if (prof) prof->begin(w == 4 ? KC_ONESWEEP32 : KC_ONESWEEP64, s);
-        var.k[mode][0]<<<pass_grid(tiles, resident_of(var), var.tma != 0), var.threads, var.smem, s>>>(a);
-        e = cudaGetLastError();
-        if (prof) prof->end(w == 4 ? KC_ONESWEEP32 : KC_ONESWEEP64, s);
-        if (e != cudaSuccess) return e;
+        const int cls = w == 4 ? KC_ONESWEEP32 : KC_ONESWEEP64;
+        if (prof) prof->begin(cls, s);
+        // the launches usually not taken are one short wave
+        const bool rare = when != nullptr && is == 1;
+        var.k[mode][0]<<<pass_grid(tiles, resident_of(var), var.tma != 0 || rare), var.threads, var.smem, s>>>(a);
+        if (prof) prof->end(cls, s);
+        return cudaGetLastError();
+    };
+    if (deep) {
+        if ((e = pass(0, true, deep, 1)) != cudaSuccess) return e;
+        if ((e = pass(1, true, deep, 0)) != cudaSuccess) return e;
+        if ((e = pass(1, false, deep, 1)) != cudaSuccess) return e;
+    } else {
+        for (int q = 0; q + 1 < D; ++q)
+            if ((e = pass(q, q == 0, nullptr, 0)) != cudaSuccess) return e;
     }
-    const void* skeys = kbuf[(P - 1) & 1];
-    const uint32_t* svals = vbuf[(P - 1) & 1];
+    if ((e = pass(D - 1, D == 1, nullptr, 0)) != cudaSuccess) return e;
+    const void* skeys = kbuf[(D - 1) & 1];
+    const uint32_t* svals = vbuf[(D - 1) & 1];
     uint32_t* chunk_start = reinterpret_cast<uint32_t*>(ws + p.off_chunks);
-    MsdChunkArgs ca{skeys, n, p.msd_chunk_rows, p.msd_chunks, (uint32_t)(8 * (ndigits - P)), chunk_start, flag};
+    MsdChunkArgs ca{skeys, n, p.msd_chunk_rows, p.msd_chunks, (uint32_t)(8 * (ndigits - P)), chunk_start, flag, deep};
     if (prof) prof->begin(KC_LOCALSORT, s);
     e = msd_chunks(ca, w, s, p.msd_cap);
     if (e == cudaSuccess) {
@@ -1316,6 +1332,7 @@ cudaError_t run_msd(const SortPlan& p, const void* const* key_cols, int order, u
         la.reverse = order == 2 ? 1 : 0;
         la.lo_bits = (uint32_t)p.msd_lo_bits;
         la.pshift = (uint32_t)(8 * (ndigits - P));
+        la.deep = deep;
         la.flag = flag;
         la.err = err;
         la.keys_out = key0_out;
@@ -1370,7 +1387,7 @@ cudaError_t run_dict(const SortPlan& p, const void* const* key_cols, int order, 
     a.status_next = nullptr;  // nothing runs after this pass when it runs
     a.status_rows = p.max_tiles;
     a.status_row_words = (uint32_t)p.max_radix;
-    a.tile_counter = counters + p.total_passes + (p.msd ? p.msd_passes : 0);
+    a.tile_counter = counters + p.total_passes + (p.msd ? p.msd_digits : 0);
     a.err = err;
     a.run_flag = word;
     a.run_when = 2;
@@ -1408,7 +1425,7 @@ cudaError_t run_sort(const SortPlan& p, const void* const* key_cols, int order, 
     if (p.msd && (e = run_msd(p, key_cols, order, perm_out, key0_out, ws, err, s, prof, perm_in)) != cudaSuccess)
         return e;
     const uint32_t* flag = reinterpret_cast<const uint32_t*>(ws + p.off_msd_flag);
-    return run_lsd(p, key_cols, order, perm_out, key0_out, ws, err, s, prof, perm_in, p.msd ? p.msd_passes : 0, flag,
+    return run_lsd(p, key_cols, order, perm_out, key0_out, ws, err, s, prof, perm_in, p.msd ? p.msd_digits : 0, flag,
                    p.msd ? msd_fallbacks : nullptr);
 }
 
