@@ -254,8 +254,8 @@ struct OnesweepCfg {
     static constexpr size_t VAL_BYTES = (size_t)TILE * 4;
     static constexpr size_t CNT_BYTES = (size_t)WARPS * RADIX * 4;
     static constexpr size_t GLOB_BYTES = (size_t)RADIX * 4;
-    // match method 3: two per-warp words per digit, the lanes holding it
-    static constexpr size_t MASK_BYTES = MATCH == 3 ? (size_t)2 * WARPS * RADIX * 4 : 0;
+    // match methods 3 and 5: two per-warp words per digit, the lanes holding it
+    static constexpr size_t MASK_BYTES = MATCH == 3 || MATCH == 5 ? (size_t)2 * WARPS * RADIX * 4 : 0;
     static constexpr size_t SMEM = KEY_BYTES + VAL_BYTES + CNT_BYTES + GLOB_BYTES + 64 + WARPS * 4 + MASK_BYTES;
     // the bulk-load variant stages the next tile in a second key / row-id buffer
     static constexpr size_t SMEM_BULK = SMEM + KEY_BYTES + VAL_BYTES;
@@ -268,6 +268,9 @@ struct OnesweepCfg {
 // ORs its bit into a per-warp shared-memory word of its digit and reads the
 // word back (two words per digit, alternating by item, so a word is cleared
 // well before it is used again).
+// 4 and 5 = match.any for every item where the warp's first one holds at most
+// kFewDigits digits (its time grows with the distinct values, that of 3 with
+// the lanes sharing one), else as 2 and as 3.
 // MINB: CTAs per SM the register allocation is sized for.
 // SEG: segmented sort of many independent row ranges (the queries of a
 // batch) in one launch.  Tiles never straddle a segment; a tile's bin bases
@@ -296,6 +299,8 @@ __device__ __forceinline__ uint32_t dict_digit(const unsigned long long* lk, con
     return 255;  // slots past the chunk: their all-ones keys rank last
 }
 
+constexpr int kFewDigits = 12;
+
 template <typename K, int BITS, int THREADS, int ITEMS, int IN_MODE, bool FINAL, int MATCH, int MINB,
           bool SEG = false, bool TMA = false, bool DICT = false>
 __global__ void __launch_bounds__(THREADS, MINB) k_onesweep(PassArgs a) {
@@ -312,7 +317,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_onesweep(PassArgs a) {
     // bulk-loaded tile, [8..11] the two buffers' mbarriers
     uint32_t* misc = bglob + RADIX;
     uint32_t* wsum = misc + 16;                                                        // [WARPS]
-    uint32_t* wmask = wsum + WARPS;  // match method 3: [2][WARPS][RADIX]
+    uint32_t* wmask = wsum + WARPS;  // match methods 3 and 5: [2][WARPS][RADIX]
     uint64_t* mbar = reinterpret_cast<uint64_t*>(misc + 8);
     K* const kbuf1 = reinterpret_cast<K*>(smem + C::SMEM);
     uint32_t* const vbuf1 = reinterpret_cast<uint32_t*>(smem + C::SMEM + C::KEY_BYTES);
@@ -373,7 +378,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_onesweep(PassArgs a) {
         // into them that follow the barrier below
         if constexpr (BULK) fence_async_smem();
         for (int i = tid; i < WARPS * RADIX; i += THREADS) wcnt[i] = 0;
-        if constexpr (MATCH == 3)
+        if constexpr (MATCH == 3 || MATCH == 5)
             for (int i = tid; i < 2 * WARPS * RADIX; i += THREADS) wmask[i] = 0;
         __syncthreads();
         const uint32_t tile = misc[2 + (it & 1)];
@@ -528,13 +533,14 @@ __global__ void __launch_bounds__(THREADS, MINB) k_onesweep(PassArgs a) {
             else if constexpr (DICT) return dict_digit(dlk, dlr, (unsigned long long)key[j]);
             else return digit_of<K, BITS>(key[j], shift);
         };
+        bool few = false;  // match method 4: few distinct digits in the warp's first item
     #pragma unroll
         for (int j = 0; j < ITEMS; ++j) {
             uint32_t d;
             if constexpr (DICT) d = dict_digit(dlk, dlr, (unsigned long long)key[j]);
             else d = digit_of<K, BITS>(key[j], shift);
             if constexpr (PACKED) dpk[j / 4] |= d << (8 * (j % 4));
-            if constexpr (MATCH == 3) {
+            if (MATCH == 3 || (MATCH == 5 && !few)) {
                 uint32_t* word = wmask + ((j & 1) * WARPS + warp) * RADIX + d;
                 atomicOr(word, 1u << lane);
                 __syncwarp();
@@ -542,8 +548,12 @@ __global__ void __launch_bounds__(THREADS, MINB) k_onesweep(PassArgs a) {
                 __syncwarp();  // every peer has read the word before its leader clears it
                 if (lane == __ffs(pm) - 1) *word = 0;
                 peers[j] = pm;
-            } else if (MATCH == 1 || (MATCH == 2 && (j & 1) == 0)) {
+                if (MATCH == 5 && j == 0) few = __popc(__ballot_sync(0xffffffffu, lane == __ffs(pm) - 1)) <= kFewDigits;
+            } else if (MATCH == 1 || MATCH == 5 || (MATCH == 2 && (j & 1) == 0) ||
+                       (MATCH == 4 && ((j & 1) == 0 || few))) {
                 peers[j] = __match_any_sync(0xffffffffu, d);
+                if (MATCH == 4 && j == 0)
+                    few = __popc(__ballot_sync(0xffffffffu, lane == __ffs(peers[0]) - 1)) <= kFewDigits;
             } else {
                 uint32_t pm = 0xffffffffu;
     #pragma unroll
@@ -850,6 +860,13 @@ const PassVariant kVariants[] = {
     make_variant<uint64_t, 8, 256, 12, 2, 2, true>(),  // 20
     make_variant<uint32_t, 8, 256, 16, 1, 2, true>(),  // 21
     make_variant<uint32_t, 8, 256, 16, 2, 2, true>(),  // 22
+    // match method chosen per warp and tile (match methods 4 and 5): the
+    // variants the library picks by size (sized_variant)
+    make_variant<uint32_t, 8, 256, 8, 4, 4>(),   // 23
+    make_variant<uint32_t, 8, 256, 12, 5, 3>(),  // 24
+    make_variant<uint32_t, 8, 256, 16, 4, 3>(),  // 25
+    make_variant<uint64_t, 8, 256, 8, 4, 4>(),   // 26
+    make_variant<uint64_t, 8, 256, 12, 5, 3>(),  // 27
 };
 constexpr int kNumVariants = (int)(sizeof(kVariants) / sizeof(kVariants[0]));
 // resident CTAs per SM of each variant's kernels (the fewest over its six)
@@ -894,7 +911,7 @@ const SegVariant kSegVariants[] = {
     make_seg_variant<8, 256, 12, 2, 2>(),   // 1
     make_seg_variant<8, 256, 16, 0, 2>(),   // 2
     make_seg_variant<11, 256, 8, 1, 2>(),   // 3
-    make_seg_variant<8, 256, 12, 2, 4>(),   // 4
+    make_seg_variant<8, 256, 12, 4, 4>(),   // 4
 };
 constexpr int kNumSegVariants = (int)(sizeof(kSegVariants) / sizeof(kSegVariants[0]));
 
@@ -953,8 +970,24 @@ bool sort_tuning_valid(const SortTuning& t) {
            t.variant64 >= 0 && t.variant64 < kNumVariants && kVariants[t.variant64].width == 8;
 }
 
+constexpr int kDefault32 = 1, kDefault64 = 2;
+
+// The default variant of a key width stands for a choice by size.  Smaller
+// tiles where the passes' latency counts (few tiles per SM), larger ones where
+// their bandwidth does; match methods 4 and 5 hold up both for spread digits
+// and where lanes share them.  LSD sort of uniform / all-equal keys on one
+// B200, fixed default -> choice: 4-byte keys 60K rows 60 / 45 -> 43 / 43 us,
+// 1M rows 97 / 63 -> 73 / 63 us, 8M rows 428 / 224 -> 318 / 221 us; 8-byte keys
+// 60K rows 91 / 87 -> 77 / 75 us, 1M rows 164 / 147 -> 145 / 117 us, 64M rows
+// 5.05 / 4.79 -> 4.40 / 3.88 ms.
+static int sized_variant(int variant, int width, uint64_t n) {
+    if (width == 4 && variant == kDefault32) return n < 750000 ? 23 : n < 3000000 ? 24 : 25;
+    if (width == 8 && variant == kDefault64) return n < 750000 ? 26 : 27;
+    return variant;
+}
+
 SortTuning default_sort_tuning() {
-    SortTuning t{1, 2, 1, kMsdDefaultMinRows};
+    SortTuning t{kDefault32, kDefault64, 1, kMsdDefaultMinRows};
     t.dict = 1;
     return t;
 }
@@ -976,7 +1009,10 @@ int msd_passes_for(uint64_t n, int width, uint32_t bucket_rows) {
     return 0;
 }
 
-SortPlan make_sort_plan(uint64_t n, const int32_t* dtypes, int nkeys, const SortTuning& tuning) {
+SortPlan make_sort_plan(uint64_t n, const int32_t* dtypes, int nkeys, const SortTuning& chosen) {
+    SortTuning tuning = chosen;
+    tuning.variant32 = sized_variant(chosen.variant32, 4, n);
+    tuning.variant64 = sized_variant(chosen.variant64, 8, n);
     SortPlan p{};
     p.n = n;
     p.nkeys = nkeys;
