@@ -13,13 +13,13 @@
 //      16 KB tile: quote parity and the two counts;
 //   2. k_csv_scan: one CTA scans the tiles: in-quote state at each tile start
 //      and the first record index of each tile;
-//   3. k_csv_records: the same masks again, now with the known state, write
-//      each record's terminator position;
+//   3. k_csv_fields: the same masks again, now with the known state, write
+//      each field's end position;
 //   4. the host reads the first rows back and classifies the columns
 //      (classify_column's rules on the first 10 values);
-//   5. k_csv_parse: one thread per record walks its fields (quote toggling,
-//      delimiter splits, as parse_rows_chunk does) and converts each field by
-//      its column's type (vdf_decimal.cuh); every lane of a warp works on the
+//   5. k_csv_parse: one thread per record walks its fields' ends, from a copy
+//      of the CTA's text in shared memory, and converts each field by its
+//      column's type (short numbers here, others in vdf_decimal.cuh); every lane of a warp works on the
 //      same column at a time, so the type branch is uniform and the column
 //      writes are coalesced; string fields record their start and length;
 //   6. strings: an offset scan per string column, then k_csv_strings copies
@@ -199,23 +199,43 @@ __global__ void __launch_bounds__(kThreads) k_csv_count(const uint8_t* __restric
 }
 
 // Pass 2 (one CTA): tile start states and first record indices; total count.
+//
+// A thread owns kScanTiles neighbouring tiles, so a round of the CTA covers
+// 8,192: the rounds are a chain of barriers (16 of 1,024 tiles for a 256 MB
+// file took 47 us; two take 29).
+constexpr int kScanTiles = 8;
+
 __global__ void __launch_bounds__(1024) k_csv_scan(const uint32_t* __restrict__ tiles, uint32_t ntiles,
                                                    uint32_t* __restrict__ tile_state, uint32_t* __restrict__ tile_first,
                                                    uint32_t* __restrict__ total) {
     __shared__ uint32_t s_w[32];
     uint32_t state = 0, first = 0;
-    for (uint32_t b = 0; b < ntiles; b += blockDim.x) {
-        const uint32_t t = b + threadIdx.x;
-        const uint32_t par = t < ntiles ? tiles[3 * t] : 0;
-        uint32_t ptot;
-        const uint32_t st = state ^ block_xor_excl(par, s_w, ptot);
-        const uint32_t cnt = t < ntiles ? (st ? tiles[3 * t + 2] : tiles[3 * t + 1]) : 0;
-        uint32_t ctot;
-        const uint32_t off = first + block_sum_excl(cnt, s_w, ctot);
-        if (t < ntiles) {
-            tile_state[t] = st;
-            tile_first[t] = off;
+    for (uint32_t b = 0; b < ntiles; b += 1024 * kScanTiles) {
+        const uint32_t t0 = b + threadIdx.x * kScanTiles;
+        uint32_t v[3 * kScanTiles];
+        uint32_t par = 0;
+#pragma unroll
+        for (int k = 0; k < kScanTiles; ++k) {
+#pragma unroll
+            for (int j = 0; j < 3; ++j) v[3 * k + j] = t0 + k < ntiles ? tiles[3 * (t0 + k) + j] : 0;
+            par ^= v[3 * k];
         }
+        uint32_t ptot;
+        uint32_t st = state ^ block_xor_excl(par, s_w, ptot);
+        uint32_t sum = 0;
+#pragma unroll
+        for (int k = 0; k < kScanTiles; ++k) {
+            const uint32_t cnt = st ? v[3 * k + 2] : v[3 * k + 1];
+            if (t0 + k < ntiles) tile_state[t0 + k] = st;
+            st ^= v[3 * k];
+            v[3 * k] = sum;  // the tile's offset within the thread's
+            sum += cnt;
+        }
+        uint32_t ctot;
+        const uint32_t off = first + block_sum_excl(sum, s_w, ctot);
+#pragma unroll
+        for (int k = 0; k < kScanTiles; ++k)
+            if (t0 + k < ntiles) tile_first[t0 + k] = off + v[3 * k];
         state ^= ptot;
         first += ctot;
     }
@@ -325,6 +345,67 @@ struct Reader {
     }
 };
 
+// The same bytes from a copy of the text in shared memory, which starts at
+// file offset `base` (a multiple of 16) and has 12 bytes to spare at its end.
+struct Staged {
+    const uint32_t* words;
+    uint32_t base;
+    __device__ __forceinline__ unsigned char get(uint64_t i) const {
+        const uint32_t k = (uint32_t)i - base;
+        return (unsigned char)(words[k >> 2] >> (8 * (k & 3)));
+    }
+    __device__ __forceinline__ uint64_t get8(uint64_t i, uint32_t avail) const {
+        const uint32_t k = (uint32_t)i - base, sh = 8 * (k & 3);
+        const uint32_t* w = words + (k >> 2);
+        const uint32_t a = w[0], b = w[1], c = w[2];
+        uint64_t v = (uint64_t)__funnelshift_r(a, b, sh) | ((uint64_t)__funnelshift_r(b, c, sh) << 32);
+        if (avail < 8) v &= (1ull << (8 * avail)) - 1;
+        return v;
+    }
+};
+
+// A field of at most eight bytes made of digits with, when `decimal`, an
+// optional '-' before them and an optional '.' among them: its digits as one
+// number (below 10^8) and how many of them follow the point.  Anything else
+// returns false.  The point is closed up, then the eight digits combine
+// pairwise in 32-bit halves: about 60 instructions, where the general readers
+// take 250 to 400 for the same field.
+template <typename Src>
+__device__ __forceinline__ bool short_field(Src& src, uint32_t fs, uint32_t len, bool decimal, uint32_t& w,
+                                            uint32_t& frac, bool& neg) {
+    if (len - 1 > 7u) return false;
+    uint64_t v = src.get8(fs, len);
+    neg = decimal && (v & 0xff) == '-';
+    if (neg) {
+        v >>= 8;
+        --len;
+    }
+    frac = 0;
+    if (decimal) {
+        const uint64_t dot =
+            ((uint64_t)eq_bytes((uint32_t)(v >> 32), 0x2e2e2e2eu) << 32) | eq_bytes((uint32_t)v, 0x2e2e2e2eu);
+        if (dot) {
+            const uint32_t at = ((uint32_t)__ffsll((long long)dot) - 1) & ~7u;  // first bit of the point's byte
+            const uint64_t below = (1ull << at) - 1;
+            v = (v & below) | ((v >> 8) & ~below);
+            --len;
+            frac = len - (at >> 3);
+        }
+    }
+    if (len == 0) return false;
+    const uint32_t pad = 64 - 8 * len;  // the digits at the top, zeros before them
+    const uint64_t t = (v ^ 0x3030303030303030ull) << pad;
+    uint32_t hi = (uint32_t)t, lo = (uint32_t)(t >> 32);  // bytes 0-3: the leading digits
+    const uint32_t over = ((hi & 0x7f7f7f7fu) + 0x76767676u) | hi | ((lo & 0x7f7f7f7fu) + 0x76767676u) | lo;
+    if (over & 0x80808080u) return false;  // a byte above 9
+    hi = ((hi * (1 + (10u << 8))) >> 8) & 0x00ff00ffu;
+    lo = ((lo * (1 + (10u << 8))) >> 8) & 0x00ff00ffu;
+    hi = (hi * (1 + (100u << 16))) >> 16;
+    lo = (lo * (1 + (100u << 16))) >> 16;
+    w = hi * 10000u + lo;
+    return true;
+}
+
 // Per-column output descriptor.
 struct CsvColDev {
     uint32_t type;  // 'd', 'u', 'b', 's', 'c'
@@ -355,14 +436,24 @@ __device__ __noinline__ double slow_field(const uint8_t* buf, uint32_t fs, uint3
     return v;
 }
 
-// Converts one field [fs, fe) of column `col` into row `row`.
-__device__ __forceinline__ void emit_field(const ParseArgs& a, Reader& rd, uint32_t fs, uint32_t fe, uint32_t col,
+// Converts one field [fs, fe) of column `d` into row `row`.
+template <typename Src>
+__device__ __forceinline__ void emit_field(const ParseArgs& a, const CsvColDev* d, Src& rd, uint32_t fs, uint32_t fe,
                                            uint32_t row, bool empty_is_na) {
-    const CsvColDev* d = a.cols + col;
-    const uint32_t type = __ldg(&d->type);
+    const uint32_t type = d->type;
     const uint32_t len = fe - fs;
     auto at = [&](uint32_t j) { return rd.get((uint64_t)fs + j); };
+    uint32_t w, frac;
+    bool neg;
     if (type == 'd') {
+        if (short_field(rd, fs, len, true, w, frac, neg)) {
+            // w < 10^8 over an exact power of ten: one correctly rounded division
+            const double p = (frac & 1 ? 10.0 : 1.0) * (frac & 2 ? 100.0 : 1.0) * (frac & 4 ? 1e4 : 1.0);
+            double v = (double)w;
+            if (frac) v = vdfdec::ddiv_rn(v, p);
+            static_cast<double*>(d->values)[row] = neg ? -v : v;
+            return;
+        }
         vdfdec::Number num;
         if (!vdfdec::scan_number_fast(rd, fs, len, num)) num = vdfdec::scan_number(at, len);
         const vdfdec::Conv cv = vdfdec::convert(num);
@@ -370,9 +461,11 @@ __device__ __forceinline__ void emit_field(const ParseArgs& a, Reader& rd, uint3
         if (cv.ambiguous) v = slow_field(a.buf, fs, len, a.err);
         static_cast<double*>(d->values)[row] = v;
     } else if (type == 'u') {
-        static_cast<uint32_t*>(d->values)[row] = vdfdec::parse_u32(at, len);
+        if (!short_field(rd, fs, len, false, w, frac, neg)) w = vdfdec::parse_u32(at, len);
+        static_cast<uint32_t*>(d->values)[row] = w;
     } else if (type == 'b') {
-        static_cast<uint8_t*>(d->values)[row] = vdfdec::parse_i32(at, len) != 0 ? 1 : 0;
+        if (!short_field(rd, fs, len, false, w, frac, neg)) w = (uint32_t)vdfdec::parse_i32(at, len);
+        static_cast<uint8_t*>(d->values)[row] = w != 0 ? 1 : 0;
     } else {
         // strings: an empty field reads "NA" (parse_rows_chunk.inl:80-81)
         const bool na = len == 0 && empty_is_na;
@@ -383,24 +476,103 @@ __device__ __forceinline__ void emit_field(const ParseArgs& a, Reader& rd, uint3
 
 // One thread per record; the threads of a CTA convert column c of their
 // records together (the same type branch, coalesced column writes), taking
-// each field's bounds from the field-end positions.
-__global__ void __launch_bounds__(kThreads) k_csv_parse(ParseArgs a) {
-    const uint32_t r = blockIdx.x * kThreads + threadIdx.x;
-    if (r >= a.records) return;
-    const uint32_t row = r + a.row_base;
-    const uint32_t* fp = a.pos + (uint64_t)r * a.ncol;
-    uint32_t fs = a.data_start;
-    if (r > 0) {
-        const uint32_t p = fp[-1];
+// each field's bounds from the field-end positions.  The CTA's records are
+// field ends and text are first copied to shared memory (`cap` bytes; a CTA
+// whose records need more reads them where they are): each field is then two
+// or three shared words wherever it starts.  Bound by instructions: 1.66M
+// records of 21 fields took 8,900 warp instructions per 32 records and 540 us
+// with windows of the text in registers and the eight-at-a-time reader for
+// every number, 3,200 and 310 us with the text alone in shared memory (each
+// field end a strided load from L2); with both, 213 us, the issue slots 70 %
+// full.
+template <typename Src>
+__device__ __forceinline__ void parse_record(const ParseArgs& a, const CsvColDev* cols, Src& rd, const uint32_t* fp,
+                                             uint32_t p, bool first, uint32_t row) {
+    uint32_t fs = p;
+    if (!first) {  // p: the terminator before the record
         fs = p + 1;
-        if (a.buf[p] == '\r' && (uint64_t)p + 1 < a.n && a.buf[p + 1] == '\n') ++fs;
+        if ((uint64_t)p + 1 < a.n && rd.get(p) == '\r' && rd.get((uint64_t)p + 1) == '\n') ++fs;
     }
-    Reader rd(a.buf, a.n);
+    uint32_t fe = fp[0];
     for (uint32_t c = 0; c < a.ncol; ++c) {
-        const uint32_t fe = fp[c];
-        emit_field(a, rd, fs, fe, c, row, true);
+        const uint32_t next = c + 1 < a.ncol ? fp[c + 1] : 0u;  // on its way during this field
+        emit_field(a, cols + c, rd, fs, fe, row, true);
         fs = fe + 1;
+        fe = next;
+        __syncwarp();  // the lanes meet again after each column's branches
     }
+}
+
+__device__ __forceinline__ void copy16(uint4* dst, const uint4* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+
+constexpr uint32_t kStageCols = 64;  // column descriptors copied as well (more are read where they are)
+
+__global__ void __launch_bounds__(kThreads) k_csv_parse(ParseArgs a, uint32_t cap) {
+    extern __shared__ uint4 s_mem[];
+    __shared__ CsvColDev s_cols[kStageCols];
+    const uint32_t r0 = blockIdx.x * blockDim.x;
+    const uint32_t rows = min(blockDim.x, a.records - r0);
+    // from the terminator before the first record to the last one's end
+    const uint32_t* fp0 = a.pos + (uint64_t)r0 * a.ncol;
+    const uint32_t fields = rows * a.ncol;
+    const uint32_t from = r0 ? fp0[-1] : a.data_start;
+    const uint64_t end = min((uint64_t)fp0[fields - 1] + 1, a.n);
+    const uint32_t base = from & ~15u;
+    const uint32_t ends = (4 * fields + 15) & ~15u;  // bytes of field ends before the text
+    const bool staged = end >= base && end - base + ends <= cap;
+    if (a.ncol <= kStageCols) {
+        for (uint32_t i = threadIdx.x; i < a.ncol; i += blockDim.x) s_cols[i] = a.cols[i];
+    }
+    const CsvColDev* cols = a.ncol <= kStageCols ? s_cols : a.cols;
+    uint32_t* s_end = reinterpret_cast<uint32_t*>(s_mem);
+    uint4* s_text = s_mem + ends / 16;
+    if (staged) {
+        // whole 16-byte pieces, asynchronously (fp0 is a multiple of 32 fields
+        // into the workspace array, which is padded to 256 bytes)
+        for (uint32_t i = threadIdx.x; i < ends / 16; i += blockDim.x)
+            copy16(s_mem + i, reinterpret_cast<const uint4*>(fp0) + i);
+        const uint32_t vecs = (uint32_t)((end - base + 15) >> 4);
+        for (uint32_t i = threadIdx.x; i < vecs; i += blockDim.x) {
+            const uint64_t at = (uint64_t)base + 16ull * i;
+            if (at + 16 <= a.n) {
+                copy16(s_text + i, reinterpret_cast<const uint4*>(a.buf + at));
+            } else {
+                uint32_t x[4] = {0, 0, 0, 0};
+                for (int k = 0; k < 16; ++k)
+                    if (at + k < a.n) x[k >> 2] |= (uint32_t)__ldg(a.buf + at + k) << (8 * (k & 3));
+                s_text[i] = make_uint4(x[0], x[1], x[2], x[3]);
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    }
+    __syncthreads();
+    if (threadIdx.x >= rows) return;
+    const uint32_t r = r0 + threadIdx.x, f = threadIdx.x * a.ncol;
+    const uint32_t p = threadIdx.x ? (staged ? s_end[f - 1] : fp0[f - 1]) : from;
+    if (staged) {
+        Staged rd{reinterpret_cast<const uint32_t*>(s_text), base};
+        parse_record(a, cols, rd, s_end + f, p, r == 0, r + a.row_base);
+    } else {
+        Reader rd(a.buf, a.n);
+        parse_record(a, cols, rd, fp0 + f, p, r == 0, r + a.row_base);
+    }
+}
+
+// Records per CTA and its shared memory: the most records (32 to 256) whose
+// field ends and text, an eighth longer than the file's average, fit 36 KB
+// (six or more CTAs per SM).
+constexpr uint32_t kStageMax = 36864;
+
+uint32_t parse_rows(uint64_t text, uint32_t records, uint32_t ncol, uint32_t& cap) {
+    const uint64_t avg = text / records + 1;
+    uint32_t rows = kThreads;
+    auto want = [&](uint64_t k) { return avg * k + avg * k / 8 + 4 * ncol * k + 512; };
+    while (rows > 32 && want(rows) > kStageMax) rows >>= 1;
+    cap = (uint32_t)std::min<uint64_t>(want(rows), kStageMax) & ~15u;
+    return rows;
 }
 
 // The first line as a data row (no header): field bounds from the host, an
@@ -409,7 +581,7 @@ __global__ void k_csv_first_line(ParseArgs a, const uint32_t* __restrict__ bound
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= a.ncol) return;
     Reader rd(a.buf, a.n);
-    emit_field(a, rd, bounds[2 * c], bounds[2 * c + 1], c, 0, c + 1 == a.ncol);
+    emit_field(a, a.cols + c, rd, bounds[2 * c], bounds[2 * c + 1], 0, c + 1 == a.ncol);
 }
 
 // Offsets: in-place inclusive scan of lengths at [1, nrow] per string column
@@ -440,8 +612,10 @@ __global__ void __launch_bounds__(kThreads) k_csv_off_partials(StrCols sc, uint6
     }
 }
 
-__global__ void __launch_bounds__(1024) k_csv_off_blocks(uint64_t* __restrict__ part, uint32_t nblk) {
-    // one CTA per string column: exclusive scan of the block sums
+__global__ void __launch_bounds__(1024) k_csv_off_blocks(uint64_t* __restrict__ part, uint32_t nblk,
+                                                         uint64_t* __restrict__ totals) {
+    // one CTA per string column: exclusive scan of the block sums, and their
+    // total (the column's bytes) beside the other columns' for one read-back
     __shared__ uint64_t s_w[32];
     uint64_t* p = part + (uint64_t)blockIdx.x * nblk;
     uint64_t carry = 0;
@@ -465,6 +639,7 @@ __global__ void __launch_bounds__(1024) k_csv_off_blocks(uint64_t* __restrict__ 
         if (i < nblk) p[i] = carry + wp + x - v;
         carry += tot;
     }
+    if (threadIdx.x == 0) totals[blockIdx.x] = carry;
 }
 
 __global__ void __launch_bounds__(kThreads) k_csv_off_apply(StrCols sc, uint64_t nrow, const uint64_t* __restrict__ part,
@@ -498,6 +673,7 @@ __global__ void __launch_bounds__(kThreads) k_csv_off_apply(StrCols sc, uint64_t
 
 struct StrCopy {
     const uint8_t* buf;
+    uint64_t n;
     uint64_t nrow;
     uint32_t nstr;
     const uint64_t* off[64];
@@ -505,52 +681,61 @@ struct StrCopy {
     uint8_t* bytes[64];
 };
 
-// One warp per 32 rows of one string column (blockIdx.y): the lanes walk the
-// rows' contiguous output span byte by byte (coalesced stores) and find each
-// byte's row by a binary search over the 32 row offsets held in lanes.
+// One warp per 32 rows of one string column (blockIdx.y).  The rows' bytes are
+// one contiguous span of the output; a lane writes one aligned eight-byte
+// piece of it at a time: a binary search over the 32 offsets (shared memory)
+// finds the piece's first row, then each row in it gives its bytes by three
+// loads and two shifts.  Bound by instructions, then by latency: with a search
+// per output byte the 1.66M rows of four columns (74 MB) took 270 us; four-byte
+// pieces with a byte loop where they cross rows, as most do, 295 us; this 189.
 __global__ void __launch_bounds__(kThreads) k_csv_strings(StrCopy sc) {
+    __shared__ uint32_t s_off[kThreads / 32][33], s_src[kThreads / 32][32];
     const uint32_t k = blockIdx.y;
     const int lane = threadIdx.x & 31;
     const uint64_t r0 = ((uint64_t)blockIdx.x * kThreads + threadIdx.x) & ~31ull;
     if (r0 >= sc.nrow) return;
     const uint64_t r = r0 + lane;
     const uint64_t* off = sc.off[k];
-    const uint64_t o = r < sc.nrow ? off[r] : off[sc.nrow];
-    const uint32_t s = r < sc.nrow ? sc.starts[k][r] : 0u;
-    const uint64_t o0 = __shfl_sync(0xffffffffu, o, 0);
+    const uint64_t o0 = off[r0];
     const uint64_t rend = r0 + 32 < sc.nrow ? r0 + 32 : sc.nrow;
-    const uint64_t span = off[rend] - o0;
-    uint8_t* dst = sc.bytes[k];
-    constexpr int U = 4;  // output bytes per lane per round: all U sources located, then loaded, then stored
-    for (uint64_t b = 0; b < span; b += 32 * U) {  // the same trip count in every lane
-        uint32_t src[U];
-        bool na[U];
-        uint8_t val[U];
+    const uint32_t span = (uint32_t)(off[rend] - o0);
+    uint32_t* so = s_off[threadIdx.x >> 5];
+    uint32_t* ss = s_src[threadIdx.x >> 5];
+    so[lane] = r < sc.nrow ? (uint32_t)(off[r] - o0) : span;  // rows past the end: empty
+    ss[lane] = r < sc.nrow ? sc.starts[k][r] : 0u;
+    if (lane == 0) so[32] = span;
+    __syncwarp();
+    uint8_t* dst = sc.bytes[k] + o0;
+    const uint32_t skew = (uint32_t)(reinterpret_cast<uintptr_t>(dst) & 7);
+    for (uint64_t i = 8 * lane; i < (uint64_t)skew + span; i += 256) {
+        const uint32_t first = i < skew ? 0u : (uint32_t)(i - skew);
+        const uint32_t last = i + 8 - skew < span ? (uint32_t)(i + 8 - skew) : span;
+        int j = 0;  // the largest j with so[j] <= first
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const uint64_t d = b + (uint64_t)u * 32 + lane;
-            const uint64_t at = o0 + (d < span ? d : span - 1);
-            // largest j with off[r0 + j] <= at (lanes past the end hold the end offset)
-            int j = 0;
-#pragma unroll
-            for (int step = 16; step; step >>= 1) {
-                const uint64_t oj = __shfl_sync(0xffffffffu, o, j + step);
-                if (oj <= at) j += step;
+        for (int step = 16; step; step >>= 1)
+            if (so[j + step] <= first) j += step;
+        uint64_t out = 0;
+        for (uint32_t b = first; b < last;) {
+            uint32_t next = so[j + 1];
+            while (next <= b) next = so[++j + 1];  // empty rows (so[32] = span > b ends it)
+            const uint32_t len = min(next, last) - b, in = b - so[j], from = ss[j] + in;
+            uint64_t v = 0;
+            if (ss[j] == 0xffffffffu) {
+                v = 0x414eu >> (8 * in);  // "NA"
+            } else if ((uint64_t)(from & ~3u) + 12 <= sc.n) {
+                const uint32_t* w = reinterpret_cast<const uint32_t*>(sc.buf + (from & ~3u));
+                const uint32_t sh = 8 * (from & 3), w0 = __ldg(w), w1 = __ldg(w + 1), w2 = __ldg(w + 2);
+                v = (uint64_t)__funnelshift_r(w0, w1, sh) | ((uint64_t)__funnelshift_r(w1, w2, sh) << 32);
+            } else {
+                for (uint32_t k8 = 0; k8 < len; ++k8) v |= (uint64_t)__ldg(sc.buf + from + k8) << (8 * k8);
             }
-            const uint64_t oj = __shfl_sync(0xffffffffu, o, j);
-            const uint32_t sj = __shfl_sync(0xffffffffu, s, j);
-            const uint32_t i = (uint32_t)(at - oj);
-            na[u] = sj == 0xffffffffu;
-            src[u] = na[u] ? i : sj + i;  // for "NA": the byte's index in "NA"
+            if (len < 8) v &= (1ull << (8 * len)) - 1;
+            out |= v << (8 * (b - first));
+            b += len;
         }
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            val[u] = na[u] ? (src[u] ? 'A' : 'N') : __ldg(sc.buf + src[u]);
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const uint64_t d = b + (uint64_t)u * 32 + lane;
-            if (d < span) dst[o0 + d] = val[u];
-        }
+        if (last - first == 8) *reinterpret_cast<uint64_t*>(dst + first) = out;
+        else
+            for (uint32_t b = first; b < last; ++b) dst[b] = (uint8_t)(out >> (8 * (b - first)));
     }
 }
 
@@ -838,6 +1023,7 @@ vdf_status csv_read_locked(vdf_ctx* c, const uint8_t* dbuf, const uint8_t* hbuf,
             str_cols.push_back(k);
         }
     }
+    static_assert(kPinnedWords >= 64, "string totals");
     if (str_cols.size() > 64) return fail(c, VDF_ERR_UNSUPPORTED, "%zu string columns (limit 64)", str_cols.size());
     // ---- outputs: values, string offsets and starts, column descriptors
     std::vector<size_t> o_val(ncol, 0), o_off(ncol, 0), o_start(ncol, 0);
@@ -859,6 +1045,8 @@ vdf_status csv_read_locked(vdf_ctx* c, const uint8_t* dbuf, const uint8_t* hbuf,
     size_t o_part = total;
     const uint32_t nblk = (uint32_t)((nrow + kScanRows - 1) / kScanRows);
     total += align256(8 * (size_t)nblk * (str_cols.empty() ? 1 : str_cols.size()) + 8);
+    const size_t o_tot = total;
+    total += align256(8 * str_cols.size());
     e = table_alloc(c->device, &t->block, total, s, t->pooled);
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -910,29 +1098,35 @@ vdf_status csv_read_locked(vdf_ctx* c, const uint8_t* dbuf, const uint8_t* hbuf,
     pa.err = err_word(c);
     begin();
     if (!header) k_csv_first_line<<<grid_of(ncol, 128), 128, 0, s>>>(pa, dbounds);
-    if (records) k_csv_parse<<<grid_of(records, kThreads), kThreads, 0, s>>>(pa);
+    if (records) {
+        uint32_t cap;
+        const uint32_t rows = parse_rows(n - data_start, records, ncol, cap);
+        k_csv_parse<<<grid_of(records, rows), rows, cap + 16, s>>>(pa, cap);
+    }
     end();
     c->launches += (header ? 0 : 1) + (records ? 1 : 0);
     // ---- string offsets
     StrCols sc;
     for (size_t k = 0; k < str_cols.size(); ++k) sc.off[k] = t->offsets[str_cols[k]];
     uint64_t* part = reinterpret_cast<uint64_t*>(t->block + o_part);
+    uint64_t* totals = reinterpret_cast<uint64_t*>(t->block + o_tot);
     if (!str_cols.empty() && nrow) {
         const dim3 g(nblk, (unsigned)str_cols.size());
         begin();
         k_csv_off_partials<<<g, kThreads, 0, s>>>(sc, nrow, part, nblk);
-        k_csv_off_blocks<<<(unsigned)str_cols.size(), 1024, 0, s>>>(part, nblk);
+        k_csv_off_blocks<<<(unsigned)str_cols.size(), 1024, 0, s>>>(part, nblk, totals);
         k_csv_off_apply<<<g, kThreads, 0, s>>>(sc, nrow, part, nblk);
         end();
         c->launches += 3;
     } else {
         for (size_t k = 0; k < str_cols.size(); ++k) cudaMemsetAsync(t->offsets[str_cols[k]], 0, 8, s);
     }
-    // string totals and the first bad record
-    std::vector<uint64_t> sums(str_cols.size() + 1, 0);
-    e = cudaMemcpyAsync(&sums[0], bad, 8, cudaMemcpyDeviceToHost, s);
-    for (size_t k = 0; k < str_cols.size() && e == cudaSuccess; ++k)
-        e = cudaMemcpyAsync(&sums[k + 1], t->offsets[str_cols[k]] + nrow, 8, cudaMemcpyDeviceToHost, s);
+    // string totals, by one copy into pinned memory
+    uint64_t* sums = &c->host_pinned[0];
+    std::memset(sums, 0, 8 * str_cols.size());
+    e = cudaSuccess;
+    if (!str_cols.empty() && nrow)
+        e = cudaMemcpyAsync(sums, totals, 8 * str_cols.size(), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {
         table_free(t->block, t->pooled);
@@ -943,8 +1137,8 @@ vdf_status csv_read_locked(vdf_ctx* c, const uint8_t* dbuf, const uint8_t* hbuf,
         std::vector<size_t> o_str(str_cols.size());
         for (size_t k = 0; k < str_cols.size(); ++k) {
             o_str[k] = stotal;
-            stotal += align256(sums[k + 1] ? sums[k + 1] : 1);
-            t->str_bytes[str_cols[k]] = sums[k + 1];
+            stotal += align256(sums[k] ? sums[k] : 1);
+            t->str_bytes[str_cols[k]] = sums[k];
         }
         e = table_alloc(c->device, &t->sblock, stotal, s, t->spooled);
         if (e != cudaSuccess) {
@@ -954,6 +1148,7 @@ vdf_status csv_read_locked(vdf_ctx* c, const uint8_t* dbuf, const uint8_t* hbuf,
         }
         StrCopy cp;
         cp.buf = dbuf;
+        cp.n = n;
         cp.nrow = nrow;
         cp.nstr = (uint32_t)str_cols.size();
         for (size_t k = 0; k < str_cols.size(); ++k) {

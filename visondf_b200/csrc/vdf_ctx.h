@@ -136,7 +136,9 @@ inline vdf::Profiler* prof_of(vdf_ctx* c) { return c->profiling ? &c->prof : nul
 
 constexpr size_t kSmallGroups = 64;  // offset in dev_small of the group-by words (vdf::DictAggWords)
 constexpr size_t kMirrorBytes = kSmallGroups + sizeof(vdf::DictAggWords);
-constexpr size_t kPinnedBytes = 8 * sizeof(uint64_t) + (kMirrorBytes + 63) / 64 * 64;
+constexpr size_t kPinnedWords = 64;  // a CSV read's string totals take up to this many from the start
+constexpr size_t kPinnedMirror = 8 * sizeof(uint64_t) + (kMirrorBytes + 63) / 64 * 64;
+constexpr size_t kPinnedBytes = kPinnedMirror > 8 * kPinnedWords ? kPinnedMirror : 8 * kPinnedWords;
 inline uint32_t* err_word(vdf_ctx* c) { return reinterpret_cast<uint32_t*>(c->dev_small); }
 inline uint64_t* count_word(vdf_ctx* c) { return reinterpret_cast<uint64_t*>(c->dev_small + 8); }
 inline uint32_t* tie_word(vdf_ctx* c) { return reinterpret_cast<uint32_t*>(c->dev_small + 16); }
