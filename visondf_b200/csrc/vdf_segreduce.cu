@@ -227,7 +227,9 @@ constexpr int kSubTiles = kSegThreads * kWideItems / kSegTile;  // 4
 constexpr int kWarpsPerSub = kSegThreads / 32 / kSubTiles;      // 2
 
 template <int NK, int NV, int VCP = 0, int KWP = 0>
-__global__ void __launch_bounds__(kSegThreads) k_seg_tiles_wide(SegArgs a, Agg<NV>* tile_agg, uint32_t tiles) {
+__global__ void __launch_bounds__(kSegThreads) k_seg_tiles_wide(SegArgs a, Agg<NV>* tile_agg, uint32_t tiles,
+                                                                uint32_t* done) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *done = 0;  // for k_seg_scan
     constexpr int ITEMS = kWideItems, WARPS = kSegThreads / 32;
     __shared__ Agg<NV> s_warp[WARPS];
     __shared__ uint32_t s_heads[WARPS];
@@ -326,10 +328,11 @@ __global__ void __launch_bounds__(kSegThreads) k_seg_tiles_wide(SegArgs a, Agg<N
 }
 
 // ---- phase 2: exclusive prefixes of the tile aggregates ----------------------
-// Level 1: each CTA scans kScanTiles consecutive tile aggregates in place
-// (exclusive, within the CTA) and writes the CTA total; level 2: one CTA
-// turns the CTA totals into exclusive prefixes.  The emit pass combines the
-// two.
+// Each CTA scans kScanTiles consecutive tile aggregates in place (exclusive,
+// within the CTA) and writes the CTA total; the CTA that finishes last (a
+// counter the tile pass clears) turns the totals into exclusive prefixes.  The
+// emit pass combines the two levels.  Latency bound: as a launch of its own
+// the second level cost 3 us and a launch gap per group-by, whatever the size.
 constexpr int kScanTiles = 256;
 
 template <int NV>
@@ -353,31 +356,34 @@ __device__ __forceinline__ Agg<NV> block_exclusive_scan(Agg<NV> x, Agg<NV>* s_wa
 }
 
 template <int NV>
-__global__ void __launch_bounds__(kScanTiles) k_seg_scan1(const SegArgs a, Agg<NV>* tile_agg, Agg<NV>* block_tot,
-                                                          uint32_t tiles) {
+__global__ void __launch_bounds__(kScanTiles) k_seg_scan(const SegArgs a, Agg<NV>* tile_agg, Agg<NV>* block_tot,
+                                                         uint32_t tiles, uint32_t* done) {
     __shared__ Agg<NV> s_warp[kScanTiles / 32];
+    __shared__ bool s_last;
     int vc[NV > 0 ? NV : 1];
 #pragma unroll
     for (int v = 0; v < NV; ++v) vc[v] = vclass(a.val[v].dtype);
-    const uint32_t t = blockIdx.x * kScanTiles + threadIdx.x;
+    const uint32_t t = blockIdx.x * kScanTiles + threadIdx.x, blocks = gridDim.x;
     const Agg<NV> x = t < tiles ? tile_agg[t] : agg_identity<NV>();
     Agg<NV> total;
     const Agg<NV> ex = block_exclusive_scan(x, s_warp, vc, total);
     if (t < tiles) tile_agg[t] = ex;
-    if (threadIdx.x == 0) block_tot[blockIdx.x] = total;
-}
-
-template <int NV>
-__global__ void __launch_bounds__(kScanTiles) k_seg_scan2(const SegArgs a, Agg<NV>* block_tot, uint32_t blocks) {
-    __shared__ Agg<NV> s_warp[kScanTiles / 32];
-    int vc[NV > 0 ? NV : 1];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) vc[v] = vclass(a.val[v].dtype);
+    if (blocks == 1) {
+        if (threadIdx.x == 0) block_tot[0] = agg_identity<NV>();
+        return;
+    }
+    if (threadIdx.x == 0) {
+        block_tot[blockIdx.x] = total;
+        __threadfence();
+        s_last = atomicAdd(done, 1u) == blocks - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
     const uint32_t per = (blocks + kScanTiles - 1) / kScanTiles;
     const uint32_t b0 = min(blocks, threadIdx.x * per), b1 = min(blocks, b0 + per);
     Agg<NV> acc = agg_identity<NV>();
     for (uint32_t b = b0; b < b1; ++b) acc = agg_combine(acc, block_tot[b], vc);
-    Agg<NV> total;
     Agg<NV> run = block_exclusive_scan(acc, s_warp, vc, total);
     for (uint32_t b = b0; b < b1; ++b) {
         const Agg<NV> cur = block_tot[b];
@@ -676,8 +682,9 @@ __global__ void __launch_bounds__(kSegThreads, (NV >= 3 ? 2 : 4))
 }
 
 template <int NK, int NV>
-cudaError_t seg_run(const SegArgs& a, unsigned char* aggs, uint32_t tiles, cudaStream_t s, Profiler* prof) {
-    Agg<NV>* ta = reinterpret_cast<Agg<NV>*>(aggs);
+cudaError_t seg_run(const SegArgs& a, unsigned char* ws, uint32_t tiles, cudaStream_t s, Profiler* prof) {
+    uint32_t* done = reinterpret_cast<uint32_t*>(ws);
+    Agg<NV>* ta = reinterpret_cast<Agg<NV>*>(ws + 256);
     const uint32_t blocks = (tiles + kScanTiles - 1) / kScanTiles;
     Agg<NV>* bt = ta + tiles;
     if (prof) prof->begin(KC_SEGREDUCE, s);
@@ -690,28 +697,27 @@ cudaError_t seg_run(const SegArgs& a, unsigned char* aggs, uint32_t tiles, cudaS
     if constexpr (NK == 2 && NV == 2) {
         launched_tiles = true;
         if (kwp == 0x48)
-            k_seg_tiles_wide<NK, NV, 1, 0x48><<<wide_grid, kSegThreads, 0, s>>>(a, ta, tiles);
+            k_seg_tiles_wide<NK, NV, 1, 0x48><<<wide_grid, kSegThreads, 0, s>>>(a, ta, tiles, done);
         else if (kwp == 0x84)
-            k_seg_tiles_wide<NK, NV, 1, 0x84><<<wide_grid, kSegThreads, 0, s>>>(a, ta, tiles);
+            k_seg_tiles_wide<NK, NV, 1, 0x84><<<wide_grid, kSegThreads, 0, s>>>(a, ta, tiles, done);
         else if (kwp == 0x44)
-            k_seg_tiles_wide<NK, NV, 1, 0x44><<<wide_grid, kSegThreads, 0, s>>>(a, ta, tiles);
+            k_seg_tiles_wide<NK, NV, 1, 0x44><<<wide_grid, kSegThreads, 0, s>>>(a, ta, tiles, done);
         else
             launched_tiles = false;
     }
     if (!launched_tiles) {
         if constexpr (NV == 2) {
-            if (fixed) k_seg_tiles_wide<NK, NV, 1><<<wide_grid, kSegThreads, 0, s>>>(a, ta, tiles);
-            else k_seg_tiles_wide<NK, NV, 0><<<wide_grid, kSegThreads, 0, s>>>(a, ta, tiles);
+            if (fixed) k_seg_tiles_wide<NK, NV, 1><<<wide_grid, kSegThreads, 0, s>>>(a, ta, tiles, done);
+            else k_seg_tiles_wide<NK, NV, 0><<<wide_grid, kSegThreads, 0, s>>>(a, ta, tiles, done);
         } else {
-            k_seg_tiles_wide<NK, NV, 0><<<wide_grid, kSegThreads, 0, s>>>(a, ta, tiles);
+            k_seg_tiles_wide<NK, NV, 0><<<wide_grid, kSegThreads, 0, s>>>(a, ta, tiles, done);
         }
     }
     if (prof) prof->end(KC_SEGREDUCE, s);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (prof) prof->begin(KC_SEGSCAN, s);
-    k_seg_scan1<NV><<<blocks, kScanTiles, 0, s>>>(a, ta, bt, tiles);
-    k_seg_scan2<NV><<<1, kScanTiles, 0, s>>>(a, bt, blocks);
+    k_seg_scan<NV><<<blocks, kScanTiles, 0, s>>>(a, ta, bt, tiles, done);
     if (prof) prof->end(KC_SEGSCAN, s);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (prof) prof->begin(KC_SEGEMIT, s);
@@ -749,13 +755,13 @@ cudaError_t seg_attrs() {
 }
 
 template <int NK>
-cudaError_t seg_run_nv(const SegArgs& a, unsigned char* aggs, uint32_t tiles, cudaStream_t s, Profiler* prof) {
+cudaError_t seg_run_nv(const SegArgs& a, unsigned char* ws, uint32_t tiles, cudaStream_t s, Profiler* prof) {
     switch (a.nvals) {
-    case 0: return seg_run<NK, 0>(a, aggs, tiles, s, prof);
-    case 1: return seg_run<NK, 1>(a, aggs, tiles, s, prof);
-    case 2: return seg_run<NK, 2>(a, aggs, tiles, s, prof);
-    case 3: return seg_run<NK, 3>(a, aggs, tiles, s, prof);
-    default: return seg_run<NK, 4>(a, aggs, tiles, s, prof);
+    case 0: return seg_run<NK, 0>(a, ws, tiles, s, prof);
+    case 1: return seg_run<NK, 1>(a, ws, tiles, s, prof);
+    case 2: return seg_run<NK, 2>(a, ws, tiles, s, prof);
+    case 3: return seg_run<NK, 3>(a, ws, tiles, s, prof);
+    default: return seg_run<NK, 4>(a, ws, tiles, s, prof);
     }
 }
 
@@ -781,7 +787,7 @@ cudaError_t prepare_segreduce_kernels() {
     return seg_attrs<4>();
 }
 
-// [256 B][tile aggregates][CTA totals of the level-1 scan]
+// [256 B: the scan's counter][tile aggregates][CTA totals of the scan]
 size_t segreduce_workspace_bytes(uint64_t n, int nvals) {
     const size_t tiles = seg_tiles(n);
     return 256 + (tiles + (tiles + kScanTiles - 1) / kScanTiles) * agg_bytes(nvals);
@@ -795,12 +801,12 @@ cudaError_t run_segreduce(SegArgs a, unsigned char* ws, cudaStream_t s, Profiler
     const uint32_t tiles = seg_tiles(a.n);
     cudaError_t e;
     switch (a.nkeys) {
-    case 1: e = seg_run_nv<1>(a, ws + 256, tiles, s, prof); break;
-    case 2: e = seg_run_nv<2>(a, ws + 256, tiles, s, prof); break;
-    case 3: e = seg_run_nv<3>(a, ws + 256, tiles, s, prof); break;
-    default: e = seg_run_nv<4>(a, ws + 256, tiles, s, prof); break;
+    case 1: e = seg_run_nv<1>(a, ws, tiles, s, prof); break;
+    case 2: e = seg_run_nv<2>(a, ws, tiles, s, prof); break;
+    case 3: e = seg_run_nv<3>(a, ws, tiles, s, prof); break;
+    default: e = seg_run_nv<4>(a, ws, tiles, s, prof); break;
     }
-    if (launches) *launches += 4;
+    if (launches) *launches += 3;
     return e;
 }
 
