@@ -98,6 +98,7 @@ __global__ void __launch_bounds__(512) k_digit_hist(HistArgs a) {
 __global__ void __launch_bounds__(256) k_hist_scan(ScanArgs a) {
     constexpr int PER = kMaxRadix / 256;
     __shared__ uint32_t warp_tot[8];
+    wait_for_launch_before();
     if (a.run_flag && *a.run_flag != 1) return;  // conditional launch (the LSD fallback) not taken
     const uint32_t radix = a.radix[blockIdx.x];
     const uint32_t* h = a.hist + a.off[blockIdx.x];
@@ -326,13 +327,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_onesweep(PassArgs a) {
     uint8_t* const ex_dig = smem + C::SMEM + sizeof(DictLut);  // DICT: digits beside the exchanged keys
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // The next pass may take its place on the SMs once all of this one's CTAs
-    // have theirs; it waits here for this one's results (no-ops where the
-    // launch before or after is an ordinary one).
-    if constexpr (!SEG) {
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-        asm volatile("griddepcontrol.launch_dependents;");
-    }
+    if constexpr (!SEG) wait_for_launch_before();
     // A conditional pass not taken returns before touching anything; the
     // flag was written by an earlier launch, so every thread reads the same.
     if (a.run_flag && *a.run_flag != a.run_when) return;
@@ -1141,24 +1136,6 @@ int sort_launches(const SortPlan& p) {
 }
 
 namespace {
-// Launches one pass; `after_pass`: the launch before it on this stream was a
-// pass too, so the two may overlap at their edges (the kernel's comment).
-// At 60,000 rows a pass is 6 us of work and the gap to the next about 1.3.
-cudaError_t launch_pass(const PassVariant& var, int mode, bool fin, uint32_t grid, const PassArgs& a, cudaStream_t s,
-                        bool after_pass) {
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3((unsigned)var.threads);
-    cfg.dynamicSmemBytes = var.smem;
-    cfg.stream = s;
-    cfg.attrs = &attr;
-    cfg.numAttrs = after_pass ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, var.k[mode][fin ? 1 : 0], a);
-}
-
 // The LSD passes over all keys (first_g: global index of the first pass, for
 // tile counters and status parity; run_flag: conditional launches).
 cudaError_t run_lsd(const SortPlan& p, const void* const* key_cols, int order, uint32_t* perm_out, void* key0_out,
@@ -1216,9 +1193,9 @@ cudaError_t run_lsd(const SortPlan& p, const void* const* key_cols, int order, u
         if (prof) prof->end(run_flag ? KC_FALLBACK : KC_HIST, s);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         if (prof) prof->begin(run_flag ? KC_FALLBACK : KC_SCAN, s);
-        k_hist_scan<<<p.total_passes, 256, 0, s>>>(sc);
+        e = launch_after(k_hist_scan, (uint32_t)p.total_passes, 256, 0, s, sc);
         if (prof) prof->end(run_flag ? KC_FALLBACK : KC_SCAN, s);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        if (e != cudaSuccess) return e;
     }
 
     const int last_g = first_g + p.total_passes - 1;
@@ -1280,7 +1257,7 @@ cudaError_t run_lsd(const SortPlan& p, const void* const* key_cols, int order, u
             a.ntiles = tiles;
             const uint32_t grid = pass_grid(tiles, resident_of(var), var.tma || run_flag != nullptr);
             if (prof) prof->begin(cls, s);
-            e = launch_pass(var, mode, fin, grid, a, s, g > first_g);
+            e = launch_after(var.k[mode][fin ? 1 : 0], grid, var.threads, var.smem, s, a);
             if (prof) prof->end(cls, s);
             if (e != cudaSuccess) return e;
             kcur = kn;

@@ -229,6 +229,7 @@ constexpr int kWarpsPerSub = kSegThreads / 32 / kSubTiles;      // 2
 template <int NK, int NV, int VCP = 0, int KWP = 0>
 __global__ void __launch_bounds__(kSegThreads) k_seg_tiles_wide(SegArgs a, Agg<NV>* tile_agg, uint32_t tiles,
                                                                 uint32_t* done) {
+    wait_for_launch_before();
     if (blockIdx.x == 0 && threadIdx.x == 0) *done = 0;  // for k_seg_scan
     constexpr int ITEMS = kWideItems, WARPS = kSegThreads / 32;
     __shared__ Agg<NV> s_warp[WARPS];
@@ -360,6 +361,7 @@ __global__ void __launch_bounds__(kScanTiles) k_seg_scan(const SegArgs a, Agg<NV
                                                          uint32_t tiles, uint32_t* done) {
     __shared__ Agg<NV> s_warp[kScanTiles / 32];
     __shared__ bool s_last;
+    wait_for_launch_before();
     int vc[NV > 0 ? NV : 1];
 #pragma unroll
     for (int v = 0; v < NV; ++v) vc[v] = vclass(a.val[v].dtype);
@@ -498,6 +500,7 @@ __global__ void __launch_bounds__(kSegThreads, (NV >= 3 ? 2 : 4))
     seg_setup<NK, NV>(a, vc, kw);
     fix_classes<NV, VCP>(vc);
     fix_widths<NK, KWP>(kw);
+    wait_for_launch_before();
     // groups that start before the CTA's rows, and in them where that is known
     const uint32_t H = block_prefix[t0 / kScanTiles].heads + tile_prefix[t0].heads;
     const uint32_t known = t1 < tiles ? block_prefix[t1 / kScanTiles].heads + tile_prefix[t1].heads - H : ~0u;
@@ -717,9 +720,9 @@ cudaError_t seg_run(const SegArgs& a, unsigned char* ws, uint32_t tiles, cudaStr
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (prof) prof->begin(KC_SEGSCAN, s);
-    k_seg_scan<NV><<<blocks, kScanTiles, 0, s>>>(a, ta, bt, tiles, done);
+    e = launch_after(k_seg_scan<NV>, blocks, kScanTiles, 0, s, a, ta, bt, tiles, done);
     if (prof) prof->end(KC_SEGSCAN, s);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (e != cudaSuccess) return e;
     if (prof) prof->begin(KC_SEGEMIT, s);
     constexpr size_t smem = emit_smem_bytes<NV>();
     auto emit = k_seg_emit<NK, NV, 0>;
@@ -731,9 +734,9 @@ cudaError_t seg_run(const SegArgs& a, unsigned char* ws, uint32_t tiles, cudaStr
         else if (kwp == 0x84) emit = k_seg_emit<NK, NV, 1, 0x84>;
         else if (kwp == 0x44) emit = k_seg_emit<NK, NV, 1, 0x44>;
     }
-    emit<<<wide_grid, kSegThreads, smem, s>>>(a, ta, bt, tiles);
+    e = launch_after(emit, wide_grid, kSegThreads, smem, s, a, ta, bt, tiles);
     if (prof) prof->end(KC_SEGEMIT, s);
-    return cudaGetLastError();
+    return e;
 }
 
 // Only three and four value columns need more than 48 KB (none of the
