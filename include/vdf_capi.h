@@ -140,9 +140,9 @@ vdf_status vdf_ctx_profile_reset(vdf_ctx* ctx);
 /* The radix pass is compiled in several variants (key width, threads per
  * CTA, keys per thread, digit bits, warp digit-match method: 0 = ballots,
  * 1 = match.any, 2 = both, alternating by item, 3 = shared-memory words
- * the lanes OR their bits into, 4 and 5 = match.any where a warp's rows hold
- * few digits, else as 2 and 3).  A context uses one variant per key width; the
- * default indices (1 and 2) stand for a choice by row count.  The reference
+ * the lanes OR their bits into; the last variants use match.any instead where
+ * a warp's rows hold few digits).  A context uses one variant per key width;
+ * the default indices (1 and 2) stand for a choice by row count.  The reference
  * fixes its digit width at 16 bits (RADIX_KI16, radix_sorts/details/
  * constants.inl:4) and has no tuning; the digit width, tile size and match
  * method here are chosen per size class by visondf_b200/autotune.py. */

@@ -862,7 +862,8 @@ const PassVariant kVariants[] = {
     make_variant<uint64_t, 8, 256, 12, 2, 2, true>(),  // 20
     make_variant<uint32_t, 8, 256, 16, 1, 2, true>(),  // 21
     make_variant<uint32_t, 8, 256, 16, 2, 2, true>(),  // 22
-    // match method chosen per warp and tile (match methods 4 and 5): the
+    // match method chosen per warp and tile (match methods 4 and 5, reported
+    // as 2 and 3, which they are where a warp's digits are many): the
     // variants the library picks by size (sized_variant)
     make_variant<uint32_t, 8, 256, 8, 4, 4>(),   // 23
     make_variant<uint32_t, 8, 256, 12, 5, 3>(),  // 24
@@ -963,7 +964,7 @@ bool sort_variant_info(int i, int* width, int* threads, int* items, int* bits, i
     *threads = v.threads;
     *items = v.items;
     *bits = v.bits;
-    *match = v.match;
+    *match = v.match >= 4 ? v.match - 2 : v.match;  // 4 and 5: 2 and 3, but match.any where digits are few
     return true;
 }
 
