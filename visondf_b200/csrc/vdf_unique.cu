@@ -5,7 +5,7 @@
 //   * k_unique_mark  marks those rows in a per-row keep mask (one pass over
 //                    the sorted keys, a scatter through the permutation);
 // The left join's First and Last need no order at all:
-//   * k_join_insert  puts the right rows into a hash table of 8-byte slots,
+//   * k_join_insert  puts the right rows into a hash table of {key, row} slots,
 //                    keeping each key's smallest (largest) row;
 //   * k_join_find    looks each left key up in it.
 // Aligned pairs the k-th occurrences of a key, which the sorted sides number:
